@@ -390,11 +390,12 @@ void slot_free(JobSlot& s) {
     dfree(s.d_queue);
     dfree(s.d_small);
     for (int k = 0; k < 2; k++) {
-        dfree(s.d_tkey[k]); dfree(s.d_tval[k]); dfree(s.d_fkey[k]); dfree(s.d_fval[k]);
+        dfree(s.d_tkey[k]); dfree(s.d_tval[k]);
     }
-    dfree(s.d_ttrec); dfree(s.d_tbox); dfree(s.d_tmeta); dfree(s.d_talpha); dfree(s.d_tcnt); dfree(s.d_tscan);
+    dfree(s.d_ttrec); dfree(s.d_tbox); dfree(s.d_tmeta); dfree(s.d_talpha);
+    dfree(s.d_titem); dfree(s.d_fnode); dfree(s.d_fhead);
     dfree(s.d_hist);
-    s.tsort_cap = s.tout_cap = s.frag_cap = s.hist_cap = 0;
+    s.tsort_cap = s.tout_cap = s.titem_cap = s.fnode_cap = s.fhead_cap = s.hist_cap = 0;
     dfree(s.d_items);
     dfree(s.d_surv);
     dfree(s.d_rec_of);
@@ -647,6 +648,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     e = grow(S, &S.d_vshade, &S.vshade_cap, (total_vtx + vrow_extra + 6 * ntt) * stride * 2);
     if (e) return e;
     const uint64_t fcap = std::min<uint64_t>(2 * total_px + 65536, 0x7FFFFFFFull);
+    const unsigned traster_blocks = (unsigned)c->nsm * DG_TRASTER_BLOCKS_PER_SM;
     if (ntt) {
         const uint64_t nout = 4 * ntt;
         if (S.tsort_cap < ntt) {
@@ -663,26 +665,23 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         }
         if (S.tout_cap < nout) {
             DG_CUDA(cudaStreamSynchronize(S.stream));
-            dfree(S.d_ttrec); dfree(S.d_tbox); dfree(S.d_tmeta); dfree(S.d_talpha); dfree(S.d_tcnt); dfree(S.d_tscan);
+            dfree(S.d_ttrec); dfree(S.d_tbox); dfree(S.d_tmeta); dfree(S.d_talpha);
             S.tout_cap = 0;
             if ((e = dalloc(&S.d_ttrec, nout)) || (e = dalloc(&S.d_tbox, nout)) || (e = dalloc(&S.d_tmeta, nout)) ||
-                (e = dalloc(&S.d_talpha, nout)) || (e = dalloc(&S.d_tcnt, nout)) || (e = dalloc(&S.d_tscan, nout + 1)))
+                (e = dalloc(&S.d_talpha, nout)))
                 return e;
             S.tout_cap = nout;
         }
-        if (S.frag_cap < fcap) {
-            DG_CUDA(cudaStreamSynchronize(S.stream));
-            for (int k = 0; k < 2; k++) {
-                dfree(S.d_fkey[k]);
-                dfree(S.d_fval[k]);
-            }
-            S.frag_cap = 0;
-            for (int k = 0; k < 2; k++) {
-                if ((e = dalloc(&S.d_fkey[k], fcap)) || (e = dalloc(&S.d_fval[k], fcap))) return e;
-            }
-            S.frag_cap = fcap;
+        e = grow(S, &S.d_titem, &S.titem_cap, nout + total_px / 64 + 65536);
+        if (e) return e;
+        e = grow(S, &S.d_fnode, &S.fnode_cap, dg_frag_nodes(fcap, traster_blocks));
+        if (e) return e;
+        if (S.fhead_cap < total_px) {
+            e = grow(S, &S.d_fhead, &S.fhead_cap, total_px);
+            if (e) return e;
+            DG_CUDA(cudaMemsetAsync(S.d_fhead, 0, S.fhead_cap * sizeof(uint32_t), S.stream));
         }
-        const uint64_t tiles = (std::max(ntt, fcap) + DG_SORT_TILE - 1) / DG_SORT_TILE;
+        const uint64_t tiles = (ntt + DG_SORT_TILE - 1) / DG_SORT_TILE;
         e = grow(S, &S.d_hist, &S.hist_cap, 256 * tiles);
         if (e) return e;
     }
@@ -765,19 +764,19 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         for (int k = 0; k < 2; k++) {
             job.tkey[k] = S.d_tkey[k];
             job.tval[k] = S.d_tval[k];
-            job.fkey[k] = S.d_fkey[k];
-            job.fval[k] = S.d_fval[k];
         }
         job.ttrec = S.d_ttrec;
         job.tbox = S.d_tbox;
         job.tmeta = S.d_tmeta;
         job.talpha = S.d_talpha;
-        job.tcnt = S.d_tcnt;
-        job.tscan = S.d_tscan;
+        job.titem = S.d_titem;
+        job.titem_cap = (uint32_t)std::min<size_t>(S.titem_cap, 0xFFFFFFF0ull);
+        job.fnode = S.d_fnode;
+        job.fnode_cap = (uint32_t)std::min<size_t>(S.fnode_cap, 0xFFFFFFF0ull);
+        job.fhead = S.d_fhead;
         job.sort_hist = S.d_hist;
         job.hist_tiles = (uint32_t)(S.hist_cap / 256);
-        // radix digits: the painter's keys are (mesh << 32 | distance key), the
-        // fragment keys (pixel << 32 | frame-local transparent key)
+        // radix digits of the painter's keys (mesh << 32 | distance key)
         auto bits = [](uint64_t v) {
             uint32_t b = 0;
             while (v) {
@@ -793,11 +792,10 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         add(p.tsort_shift, p.n_tsort, 0, 32);
         add(p.tsort_shift, p.n_tsort, 32, bits(tmesh_total - 1));
         if (p.n_tsort & 1u) p.tsort_shift[p.n_tsort++] = 56;  // even pass count: the result lands in buffer 0
-        add(p.fsort_shift, p.n_fsort, 0, bits(4 * max_frame_tt - 1));
-        add(p.fsort_shift, p.n_fsort, 32, bits(total_px - 1));
-        if (p.n_fsort & 1u) p.fsort_shift[p.n_fsort++] = 56;
+        p.key_bits = bits(4 * max_frame_tt - 1);
         p.blocks = (unsigned)c->nsm * 8u;
-        B.launches += 3 * (p.n_tsort + p.n_fsort) + 6;
+        p.raster_blocks = traster_blocks;
+        B.launches += 3 * p.n_tsort + 5;
     }
     B.cfg.vertex_blocks = (unsigned)c->nsm * DG_VERTEX_BLOCKS_PER_SM;
     B.cfg.cull_blocks = (unsigned)c->nsm * S.cull_blocks_per_sm;

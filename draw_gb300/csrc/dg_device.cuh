@@ -619,6 +619,25 @@ __device__ __forceinline__ void wait_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Hands out n consecutive slots of counter c to every lane of the (converged)
+// warp with one atomic; returns this lane's first slot.
+__device__ __forceinline__ unsigned long long warp_alloc(unsigned long long* c, uint32_t n) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(FULL, incl, 31);
+    unsigned long long old = 0;
+    if (total != 0u) {
+        if (lane == 31u) old = atomicAdd(c, (unsigned long long)total);
+        old = __shfl_sync(FULL, old, 31);
+    }
+    return old + (incl - n);
+}
+
 // Rasterizes a triangle's clipped bounding box on the calling lane alone, row
 // by row (the pixel position advances without division).
 __device__ __forceinline__ void raster_box(const EdgeSet& e, float da, float db, float dc, uint32_t seq, uint32_t xlo,
@@ -1042,8 +1061,9 @@ inline unsigned grid_for(uint64_t n, unsigned cap) {
 // Programmatic dependent launch: the kernel may be scheduled while the previous
 // kernel of the stream drains; it calls wait_previous_kernel() before reading
 // anything that kernel wrote.
-template <class Arg>
-cudaError_t launch_dependent(void (*kern)(Arg), unsigned grid, unsigned block, const Arg& arg, cudaStream_t s) {
+template <class Arg, class... More>
+cudaError_t launch_dependent(void (*kern)(Arg, More...), unsigned grid, unsigned block, const Arg& arg, cudaStream_t s,
+                             More... more) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -1054,7 +1074,7 @@ cudaError_t launch_dependent(void (*kern)(Arg), unsigned grid, unsigned block, c
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, arg);
+    return cudaLaunchKernelEx(&cfg, kern, arg, more...);
 }
 
 }  // namespace

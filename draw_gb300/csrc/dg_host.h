@@ -145,12 +145,13 @@ struct JobSlot {
     uint4* d_tbox = nullptr;
     uint2* d_tmeta = nullptr;
     float* d_talpha = nullptr;
-    uint32_t* d_tcnt = nullptr;
-    unsigned long long* d_tscan = nullptr;
-    size_t tout_cap = 0;  // clip outputs the arrays above hold (tscan: one more)
-    uint64_t* d_fkey[2] = {};
-    uint32_t* d_fval[2] = {};
-    size_t frag_cap = 0;
+    size_t tout_cap = 0;  // clip outputs the arrays above hold
+    uint4* d_titem = nullptr;
+    size_t titem_cap = 0;
+    uint4* d_fnode = nullptr;
+    size_t fnode_cap = 0;
+    uint32_t* d_fhead = nullptr;  // zeroed at allocation; the fold clears what the raster sets
+    size_t fhead_cap = 0;
     uint32_t* d_hist = nullptr;
     size_t hist_cap = 0;  // entries
     uint2* d_items = nullptr;  // raster work items

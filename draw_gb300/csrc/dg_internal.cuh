@@ -231,8 +231,11 @@ struct alignas(16) DgQueueRec {
 #define DG_CNT_UNITS (6 * DG_CNT_LINE)    // work units of the queued triangles
 #define DG_CNT_SMALL (7 * DG_CNT_LINE)    // entries of the small-triangle list
 #define DG_CNT_TRECX (8 * DG_CNT_LINE)    // records handed out after the first total_tri (multi-output clips)
+#define DG_CNT_TITEM (9 * DG_CNT_LINE)    // first items of the transparent outputs
 #define DG_CNT_TFRAG (10 * DG_CNT_LINE)   // transparent fragments emitted
-#define DG_NCOUNTERS (12 * DG_CNT_LINE)   // words of the counter array (k_vertex zeroes them: <= 256)
+#define DG_CNT_TITEMX (11 * DG_CNT_LINE)  // further items of the transparent outputs
+#define DG_CNT_TSLOT (12 * DG_CNT_LINE)   // fragment nodes handed out (chunks of DG_FRAG_CHUNK)
+#define DG_NCOUNTERS (13 * DG_CNT_LINE)   // words of the counter array (k_vertex zeroes them: <= 256)
 
 struct DgJobDev {
     const DgFrameDev* frames;
@@ -271,29 +274,45 @@ struct DgJobDev {
     uint32_t* err;
     // Transparent pass (all null/zero when the job has no transparent triangle).
     uint32_t ntt;           // transparent triangles of the job
-    uint32_t fcap;          // capacity of the fragment buffers
+    uint32_t fcap;          // most transparent fragments a job may have (DG_E_LIMIT beyond)
     uint64_t* tkey[2];      // painter's sort: keys and source slots, [ntt] each
     uint32_t* tval[2];
     DgTriRec* ttrec;        // [4 ntt] records of clip outputs, 4 j + o for sorted slot j
     uint4* tbox;            // [4 ntt] (xlo, ylo, width, frame) of each output's bounding box
     uint2* tmeta;           // [4 ntt] (object rank within the frame, frame-local transparent key)
     float* talpha;          // [4 ntt] material alpha
-    uint32_t* tcnt;         // [4 ntt] bounding-box pixels of each output, 0 for none
-    unsigned long long* tscan;  // [4 ntt + 1] exclusive prefix sums of tcnt
-    uint64_t* fkey[2];      // fragments: (job-wide pixel << 32 | transparent key), output record
-    uint32_t* fval[2];
+    // Work items of the transparent raster: (output record, first unit, end unit,
+    // box pixels). The first item of every output is in [0, 4 ntt), the further
+    // ones of large boxes follow (an output whose further items do not fit has
+    // them all in its first).
+    uint4* titem;
+    uint32_t titem_cap;     // entries of titem
+    // Transparent fragments as one linked list per pixel: fhead[job-wide pixel]
+    // is the last fragment's node + 1, 0 for none (kept zero between jobs);
+    // a node is (previous node + 1, transparent key, shaded colour, alpha bits).
+    uint4* fnode;
+    uint32_t fnode_cap;     // nodes: fcap, and a partly used chunk per warp of the raster
+    uint32_t* fhead;        // [total_px]
     uint32_t* sort_hist;    // radix sort histograms, 256 per tile of DG_SORT_TILE keys
     uint32_t hist_tiles;    // tiles sort_hist has room for
 };
 
-// Launch plan of the transparent pass: the digit shifts of its two radix
-// sorts (painter's sort keys, fragment keys) and the grid of its grid-stride
-// kernels.
+// Launch plan of the transparent pass: the digit shifts of its radix sort
+// (painter's sort keys), the key bits of its fragments and its grids.
 struct DgTransparentPlan {
     uint32_t tsort_shift[8], n_tsort;  // painter's sort digits
-    uint32_t fsort_shift[8], n_fsort;  // fragment sort digits
+    uint32_t key_bits;                 // bits of a transparent key
     unsigned blocks;                   // grid of the grid-stride kernels
+    unsigned raster_blocks;            // grid of the fragment raster
 };
+// k_traster: units (DG_UNIT_PX pixels) per work item, nodes a warp takes from the
+// node array at a time, resident blocks per SM.
+#define DG_TITEM_UNITS 8u
+#define DG_FRAG_CHUNK 128u
+#define DG_TRASTER_BLOCKS_PER_SM 3u
+// Nodes for n fragments written by `blocks` 256-thread blocks: every warp may
+// leave one chunk partly used.
+constexpr uint64_t dg_frag_nodes(uint64_t n, unsigned blocks) { return n + (uint64_t)blocks * 8u * DG_FRAG_CHUNK; }
 
 // The descriptors of a small job (one frame, at most DG_INLINE_SEGS segments)
 // travel as a kernel parameter of k_vertex instead of a host-to-device copy:

@@ -200,25 +200,6 @@ __global__ void __launch_bounds__(256) k_cull(const DgJobDev job) {
 // clipping, triangle records, bounding boxes and edge functions; tiny
 // triangles are rasterized by their warp, the others are queued
 // (scene/mod.rs:1029-1063, canvas.rs:585-681).
-// Hands out n consecutive slots of counter c to every lane of the (converged)
-// warp with one atomic; returns this lane's first slot.
-__device__ __forceinline__ unsigned long long warp_alloc(unsigned long long* c, uint32_t n) {
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t incl = n;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= (uint32_t)o) incl += v;
-    }
-    const uint32_t total = __shfl_sync(FULL, incl, 31);
-    unsigned long long old = 0;
-    if (total != 0u) {
-        if (lane == 31u) old = atomicAdd(c, (unsigned long long)total);
-        old = __shfl_sync(FULL, old, 31);
-    }
-    return old + (incl - n);
-}
-
 __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
     __shared__ uint32_t s_records;  // statistics: record requests of the block
     __shared__ uint32_t s_nclip;    // clipped survivors the block deferred
