@@ -276,6 +276,7 @@ void free_object(Object& o) {
     dfree(o.d_tri_pos); dfree(o.d_tri_uv); dfree(o.d_tri_nrm); dfree(o.d_mats);
     for (int b = 0; b < 2; b++)
         for (int k = 0; k < 3; k++) dfree(o.d_tt[b][k]);
+    dfree(o.d_tmesh_off);
 }
 
 Scene* get_scene(dg_ctx* c, int32_t id) {
@@ -498,6 +499,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     segs.clear();
     uint64_t total_vtx = 0, total_tri = 0, total_tiles = 0, total_px = 0;
     uint64_t ntt = 0, tmesh_total = 0, max_frame_tt = 0;
+    uint32_t tmesh_max = 0;
     uint32_t stride = 1;
     bool any_persp = false, any_lazy = false;
     B.transparent_objects.clear();
@@ -615,6 +617,8 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
             sg.nt = o.nt;
             sg.tmesh_base = (uint32_t)tmesh_total;
             sg.obj_rank = (uint32_t)(segs.size() - f.seg_begin);
+            sg.tmesh_off = o.d_tmesh_off;
+            if (o.nt) tmesh_max = std::max(tmesh_max, o.tmesh_max);
             for (int k = 0; k < 3; k++) {
                 sg.tsrc[k] = o.d_tt[o.tcur][k];
                 sg.tdst[k] = o.d_tt[1 - o.tcur][k];
@@ -776,7 +780,6 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         job.fhead = S.d_fhead;
         job.sort_hist = S.d_hist;
         job.hist_tiles = (uint32_t)(S.hist_cap / 256);
-        // radix digits of the painter's keys (mesh << 32 | distance key)
         auto bits = [](uint64_t v) {
             uint32_t b = 0;
             while (v) {
@@ -786,16 +789,18 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
             return b;
         };
         DgTransparentPlan& p = B.cfg.tplan;
-        auto add = [](uint32_t* sh, uint32_t& np, uint32_t lo, uint32_t nbits) {
-            for (uint32_t b = 0; b < nbits; b += 8) sh[np++] = lo + b;
-        };
-        add(p.tsort_shift, p.n_tsort, 0, 32);
-        add(p.tsort_shift, p.n_tsort, 32, bits(tmesh_total - 1));
-        if (p.n_tsort & 1u) p.tsort_shift[p.n_tsort++] = 56;  // even pass count: the result lands in buffer 0
+        if (tmesh_max <= DG_TSORT_MAX) {
+            p.tsort_meshes = (uint32_t)tmesh_total;
+            for (p.tsort_pow2 = 64; p.tsort_pow2 < tmesh_max;) p.tsort_pow2 *= 2;
+        } else {
+            // radix digits of the painter's keys (mesh << 32 | distance key)
+            for (uint32_t b = 0; b < 32 + bits(tmesh_total - 1); b += 8) p.tsort_shift[p.n_tsort++] = b;
+            if (p.n_tsort & 1u) p.tsort_shift[p.n_tsort++] = 56;  // even pass count: the result lands in buffer 0
+        }
         p.key_bits = bits(4 * max_frame_tt - 1);
         p.blocks = (unsigned)c->nsm * 8u;
         p.raster_blocks = traster_blocks;
-        B.launches += 3 * p.n_tsort + 5;
+        B.launches += 3 + (p.tsort_meshes ? 1 : 3 * p.n_tsort + 2);
     }
     B.cfg.vertex_blocks = (unsigned)c->nsm * DG_VERTEX_BLOCKS_PER_SM;
     B.cfg.cull_blocks = (unsigned)c->nsm * S.cull_blocks_per_sm;
@@ -1141,6 +1146,7 @@ dg_status dg_object_create(dg_ctx* c, const float* vertices, uint64_t nv, const 
                 xnrm.push_back(make_uint4(q[6], q[7], q[8], 0u));
             }
             o.tmesh_off.push_back((uint32_t)xpos.size());
+            o.tmesh_max = std::max(o.tmesh_max, (uint32_t)md.ntri);
             continue;
         }
         for (uint64_t t = 0; t < md.ntri; t++) {
@@ -1172,7 +1178,7 @@ dg_status dg_object_create(dg_ctx* c, const float* vertices, uint64_t nv, const 
         (e = up(&o.d_tri_uv, tuv)) || (e = up(&o.d_tri_nrm, tnrm)) || (e = up(&o.d_mats, dm)) ||
         (e = up(&o.d_tt[0][0], xpos)) || (e = up(&o.d_tt[0][1], xuv)) || (e = up(&o.d_tt[0][2], xnrm)) ||
         (e = dalloc(&o.d_tt[1][0], xpos.size())) || (e = dalloc(&o.d_tt[1][1], xpos.size())) ||
-        (e = dalloc(&o.d_tt[1][2], xpos.size()))) {
+        (e = dalloc(&o.d_tt[1][2], xpos.size())) || (e = up(&o.d_tmesh_off, o.tmesh_off))) {
         free_object(o);
         return e;
     }

@@ -1062,12 +1062,12 @@ inline unsigned grid_for(uint64_t n, unsigned cap) {
 // kernel of the stream drains; it calls wait_previous_kernel() before reading
 // anything that kernel wrote.
 template <class Arg, class... More>
-cudaError_t launch_dependent(void (*kern)(Arg, More...), unsigned grid, unsigned block, const Arg& arg, cudaStream_t s,
-                             More... more) {
+cudaError_t launch_dependent_smem(void (*kern)(Arg, More...), unsigned grid, unsigned block, size_t smem, const Arg& arg,
+                                  cudaStream_t s, More... more) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1075,6 +1075,11 @@ cudaError_t launch_dependent(void (*kern)(Arg, More...), unsigned grid, unsigned
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, arg, more...);
+}
+template <class Arg, class... More>
+cudaError_t launch_dependent(void (*kern)(Arg, More...), unsigned grid, unsigned block, const Arg& arg, cudaStream_t s,
+                             More... more) {
+    return launch_dependent_smem(kern, grid, block, 0, arg, s, more...);
 }
 
 }  // namespace

@@ -86,6 +86,8 @@ struct Object {
     int tcur = 0;
     uint32_t nt = 0;
     std::vector<uint32_t> tmesh_off;
+    uint32_t* d_tmesh_off = nullptr;
+    uint32_t tmesh_max = 0;  // triangles of the largest transparent mesh
 };
 
 struct Canvas {

@@ -163,6 +163,7 @@ struct DgSegDev {
     uint32_t obj_rank;    // the object's position within its frame
     const uint4* tsrc[3];
     uint4* tdst[3];
+    const uint32_t* tmesh_off;  // first triangle of each transparent mesh of the object, then nt
 };
 
 // Edge constants of one triangle: f_k(x, y) = ((A[k]*x + B[k]*y) + C[k]) - D[k]
@@ -297,16 +298,26 @@ struct DgJobDev {
     uint32_t hist_tiles;    // tiles sort_hist has room for
 };
 
-// Launch plan of the transparent pass: the digit shifts of its radix sort
-// (painter's sort keys), the key bits of its fragments and its grids.
+// Launch plan of the transparent pass: its painter's sort, the key bits of its
+// fragments and its grids.
 struct DgTransparentPlan {
-    uint32_t tsort_shift[8], n_tsort;  // painter's sort digits
+    // Painter's sort: with every mesh at most DG_TSORT_MAX triangles, one block
+    // per mesh (tsort_meshes > 0) with tsort_pow2 keys of shared memory; else the
+    // radix sort's digits.
+    uint32_t tsort_meshes, tsort_pow2;
+    uint32_t tsort_shift[8], n_tsort;
     uint32_t key_bits;                 // bits of a transparent key
     unsigned blocks;                   // grid of the grid-stride kernels
     unsigned raster_blocks;            // grid of the fragment raster
 };
+// Largest mesh that one block sorts in shared memory (32 KB of keys, the static
+// limit with room for two blocks per SM); larger ones take the radix sort, which
+// reads and writes every key six times or more in 3-kernel passes.
+#define DG_TSORT_MAX 4096u
 // k_traster: units (DG_UNIT_PX pixels) per work item, nodes a warp takes from the
-// node array at a time, resident blocks per SM.
+// node array at a time, resident blocks per SM (with 4, a cap of 64 registers, it
+// spills; a 1280x720 frame with 19,000 transparent triangles takes 220 us against
+// 201; with 4 or 16 units per item 201 and 217 us against 197).
 #define DG_TITEM_UNITS 8u
 #define DG_FRAG_CHUNK 128u
 #define DG_TRASTER_BLOCKS_PER_SM 3u
