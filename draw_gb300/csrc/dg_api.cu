@@ -958,11 +958,8 @@ dg_status dg_ctx_destroy(dg_ctx* c) {
     slot_free(c->main);
     {
         OverlaySlot& O = c->overlay;
-        dfree(O.d_rec); dfree(O.d_box); dfree(O.d_scan); dfree(O.d_hist); dfree(O.d_cnt); dfree(O.d_rgba);
-        for (int k = 0; k < 2; k++) {
-            dfree(O.d_fkey[k]);
-            dfree(O.d_fval[k]);
-        }
+        dfree(O.d_verts); dfree(O.d_box); dfree(O.d_items); dfree(O.d_node); dfree(O.d_head); dfree(O.d_cnt);
+        dfree(O.d_rgba);
     }
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
@@ -1512,44 +1509,6 @@ struct HRect {
     }
 };
 
-// The edge set of dg_device.cuh make_edges, on the host (the same f32
-// operations; this file is compiled without contraction), as the 16 words of
-// a triangle record: A[3], B[3], C[3], D[3], den[3], tie bits.
-void host_edges(float ax, float ay, float bx, float by, float cx, float cy, float w[16]) {
-    const float px[3] = {bx, cx, ax}, py[3] = {by, cy, ay};
-    const float qx[3] = {cx, ax, bx}, qy[3] = {cy, ay, by};
-    const float vx[3] = {ax, bx, cx}, vy[3] = {ay, by, cy};
-    float A[3], B[3], C[3], D[3], den[3];
-    uint32_t tie = 0;
-    for (int k = 0; k < 3; k++) {
-        A[k] = py[k] - qy[k];
-        B[k] = qx[k] - px[k];
-        C[k] = px[k] * qy[k];
-        D[k] = qx[k] * py[k];
-    }
-    auto eval = [&](int k, float x, float y) { return ((A[k] * x + B[k] * y) + C[k]) - D[k]; };
-    for (int k = 0; k < 3; k++) {
-        den[k] = eval(k, vx[k], vy[k]);
-        if (den[k] * eval(k, -1.0f, -1.0f) > 0.0f) tie |= 1u << k;
-    }
-    bool fast = true;
-    for (int k = 0; k < 3; k++) {
-        if (std::signbit(den[k])) {
-            A[k] = -A[k];
-            B[k] = -B[k];
-            C[k] = -C[k];
-            D[k] = -D[k];
-            den[k] = -den[k];
-        }
-        fast = fast && den[k] > 0.0f && den[k] < INFINITY;
-    }
-    if (fast) tie |= DG_EDGE_FAST;
-    const float words[16] = {A[0], A[1], A[2], B[0], B[1], B[2], C[0], C[1], C[2], D[0], D[1], D[2],
-                             den[0], den[1], den[2], 0.0f};
-    std::memcpy(w, words, sizeof(words));
-    std::memcpy(w + 15, &tie, 4);
-}
-
 }  // namespace
 
 dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* verts, uint32_t n, int32_t texmap,
@@ -1563,16 +1522,15 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
     if (e) return e;
     e = sync_tex_table(c, c->main.stream);
     if (e) return e;
-    // host setup (canvas.rs:449-535): snapped centres, bounding box clipped to the
-    // screen and the clipping rectangle, edges, attributes
-    std::vector<DgTriRec> rec(n);
+    // host setup (canvas.rs:449-535): the bounding box of the snapped centres clipped
+    // to the screen and the clipping rectangle, cut into work items
     std::vector<uint4> box(n);
-    std::vector<unsigned long long> scan(n + 1);
+    std::vector<uint2> items;
     const HRect screen = HRect::from_coords(0, 0, cv->w - 1, cv->h - 1);
     unsigned long long total = 0;
     for (uint32_t t = 0; t < n; t++) {
         const float* v = verts + 24ull * t;
-        float cx[3], cy[3], words[28];
+        float cx[3], cy[3];
         for (int k = 0; k < 3; k++) {  // pos_map_center, canvas.rs:896-904
             cx[k] = std::floor(v[8 * k] + 0.5f);
             cy[k] = std::floor(v[8 * k + 1] + 0.5f);
@@ -1598,50 +1556,42 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
                                : screen;
         const HRect valid = HRect::clip(cr, drawable);
         if (valid.x + valid.w >= cv->w || valid.y + valid.h >= cv->h) return DG_E_INVALID;  // outside the canvas
-        host_edges(cx[0], cy[0], cx[1], cy[1], cx[2], cy[2], words);
-        uint32_t col[3];
-        for (int k = 0; k < 3; k++) {  // Color::Custom([r, g, b]).as_pixel(): b, g, r bytes
+        for (int k = 0; k < 3; k++) {
             const float* p = v + 8 * k;
             if (!(p[4] >= 0.0f && p[4] <= 255.0f && p[5] >= 0.0f && p[5] <= 255.0f && p[6] >= 0.0f && p[6] <= 255.0f))
                 return DG_E_INVALID;
-            col[k] = (uint32_t)(uint8_t)p[6] | ((uint32_t)(uint8_t)p[5] << 8) | ((uint32_t)(uint8_t)p[4] << 16);
         }
-        const float w4[4] = {v[2], v[10], v[18], v[7]}, w5[4] = {v[3], v[11], v[19], v[15]};
-        std::memcpy(words + 16, w4, 16);
-        std::memcpy(words + 20, w5, 16);
-        std::memcpy(words + 24, col, 12);
-        std::memcpy(words + 27, &v[23], 4);
-        std::memset(&rec[t], 0, sizeof(DgTriRec));
-        std::memcpy(&rec[t], words, sizeof(words));
-        const uint64_t bw = valid.w + 1, bh = valid.h + 1;
-        box[t] = make_uint4((uint32_t)valid.x, (uint32_t)valid.y, (uint32_t)bw, 0u);
-        scan[t] = total;
-        total += bw * bh;
+        const uint64_t npx = (valid.w + 1) * (valid.h + 1);
+        box[t] = make_uint4((uint32_t)valid.x, (uint32_t)valid.y, (uint32_t)valid.w + 1u, (uint32_t)npx);
+        total += npx;
+        if (total >= 0x7FFFFFFFull) continue;  // refused below
+        const uint32_t units = (uint32_t)((npx + DG_UNIT_PX - 1) / DG_UNIT_PX), step = dg_overlay_units(npx);
+        for (uint32_t u = 0; u < units; u += step) items.push_back(make_uint2(t, u));
     }
-    scan[n] = total;
     if (total >= 0x7FFFFFFFull) return DG_E_LIMIT;
     JobSlot& S = c->main;
     OverlaySlot& O = c->overlay;
-    auto need = [&](auto** p, size_t* cap, size_t k) -> dg_status { return grow(S, p, cap, std::max<size_t>(k, 1)); };
-    if ((e = need(&O.d_rec, &O.rec_cap, n)) || (e = need(&O.d_box, &O.box_cap, n)) ||
-        (e = need(&O.d_scan, &O.scan_cap, n + 1)) || (e = need(&O.d_fkey[0], &O.frag_cap[0], total)) ||
-        (e = need(&O.d_fkey[1], &O.frag_cap[1], total)) || (e = need(&O.d_fval[0], &O.frag_cap[2], total)) ||
-        (e = need(&O.d_fval[1], &O.frag_cap[3], total)) ||
-        (e = need(&O.d_hist, &O.hist_cap, 256 * ((total + DG_SORT_TILE - 1) / DG_SORT_TILE))) ||
-        (e = need(&O.d_cnt, &O.cnt_cap, 1)))
+    const unsigned blocks = (unsigned)c->nsm * DG_OVERLAY_BLOCKS_PER_SM;
+    if ((e = grow(S, &O.d_verts, &O.verts_cap, 6ull * n)) || (e = grow(S, &O.d_box, &O.box_cap, n)) ||
+        (e = grow(S, &O.d_items, &O.items_cap, items.size())) ||
+        (e = grow(S, &O.d_node, &O.node_cap, dg_frag_nodes(total, blocks))) || (e = grow(S, &O.d_cnt, &O.cnt_cap, 1)))
         return e;
+    if (O.head_cap < cv->w * cv->h) {
+        if ((e = grow(S, &O.d_head, &O.head_cap, cv->w * cv->h))) return e;
+        DG_CUDA(cudaMemsetAsync(O.d_head, 0, O.head_cap * sizeof(uint32_t), S.stream));
+    }
     DG_CUDA(cudaStreamSynchronize(S.stream));  // the scratch may still be read by the previous batch
-    DG_CUDA(cudaMemcpyAsync(O.d_rec, rec.data(), n * sizeof(DgTriRec), cudaMemcpyHostToDevice, S.stream));
+    DG_CUDA(cudaMemcpyAsync(O.d_verts, verts, n * 24ull * sizeof(float), cudaMemcpyHostToDevice, S.stream));
     DG_CUDA(cudaMemcpyAsync(O.d_box, box.data(), n * sizeof(uint4), cudaMemcpyHostToDevice, S.stream));
-    DG_CUDA(cudaMemcpyAsync(O.d_scan, scan.data(), (n + 1) * sizeof(unsigned long long), cudaMemcpyHostToDevice,
-                            S.stream));
+    DG_CUDA(cudaMemcpyAsync(O.d_items, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice, S.stream));
     DG_CUDA(cudaMemsetAsync(O.d_cnt, 0, sizeof(unsigned long long), S.stream));
     DgOverlayJob j;
     std::memset(&j, 0, sizeof(j));
-    j.rec = O.d_rec;
+    j.verts = O.d_verts;
     j.box = O.d_box;
-    j.scan = O.d_scan;
+    j.items = O.d_items;
     j.n = n;
+    j.nitems = (uint32_t)items.size();
     j.width = (uint32_t)cv->w;
     j.height = (uint32_t)cv->h;
     j.colour = cv->d_colour;
@@ -1655,26 +1605,13 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
     j.tex.fw = (float)tm.w;
     j.tex.fh = (float)tm.h;
     j.tex.small = dg_tex_small(tm.len, tm.w, tm.h);
-    for (int k = 0; k < 2; k++) {
-        j.fkey[k] = O.d_fkey[k];
-        j.fval[k] = O.d_fval[k];
-    }
-    j.fcap = (uint32_t)total;
-    j.hist = O.d_hist;
+    j.node = O.d_node;
+    j.node_cap = (uint32_t)std::min<size_t>(O.node_cap, 0xFFFFFFF0ull);
+    j.head = O.d_head;
     j.cnt = O.d_cnt;
     j.err = S.d_err;
-    auto bits = [](uint64_t v) {
-        uint32_t b = 0;
-        while (v) {
-            b++;
-            v >>= 1;
-        }
-        return b;
-    };
-    for (uint32_t b = 0; b < bits(n - 1); b += 8) j.sort_shift[j.n_sort++] = b;
-    for (uint32_t b = 0; b < bits(cv->w * cv->h - 1); b += 8) j.sort_shift[j.n_sort++] = 32 + b;
-    if (j.n_sort & 1u) j.sort_shift[j.n_sort++] = 56;  // even pass count: the result lands in buffer 0
-    DG_CUDA(dg_launch_overlay(j, (unsigned)c->nsm * 8u, S.stream));
+    for (uint32_t b = n - 1; b; b >>= 1) j.key_bits++;
+    DG_CUDA(dg_launch_overlay(j, blocks, S.stream));
     return DG_OK;
 }
 

@@ -197,17 +197,16 @@ struct JobSlot {
 namespace dgh {
 // Scratch of dg_canvas_draw_triangles_2d (grow-only, on the context stream).
 struct OverlaySlot {
-    DgTriRec* d_rec = nullptr;
-    size_t rec_cap = 0;
+    float4* d_verts = nullptr;
+    size_t verts_cap = 0;
     uint4* d_box = nullptr;
     size_t box_cap = 0;
-    unsigned long long* d_scan = nullptr;
-    size_t scan_cap = 0;
-    uint64_t* d_fkey[2] = {};
-    uint32_t* d_fval[2] = {};
-    size_t frag_cap[4] = {};
-    uint32_t* d_hist = nullptr;
-    size_t hist_cap = 0;
+    uint2* d_items = nullptr;
+    size_t items_cap = 0;
+    uint4* d_node = nullptr;
+    size_t node_cap = 0;
+    uint32_t* d_head = nullptr;  // zeroed at allocation; the fold clears what the raster sets
+    size_t head_cap = 0;
     unsigned long long* d_cnt = nullptr;
     size_t cnt_cap = 0;
     uint32_t* d_rgba = nullptr;  // staging of dg_canvas_read_rgba

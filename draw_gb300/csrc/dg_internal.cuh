@@ -376,28 +376,34 @@ bool dg_timeline_copy(unsigned long long* out, cudaStream_t s, cudaError_t* err)
 cudaError_t dg_launch_transparent(int part, const DgJobDev& job, const DgTransparentPlan& plan, cudaStream_t s);
 
 // One batch of 2D overlay triangles (Canvas::draw_triangle, canvas.rs:435-575)
-// drawn into one canvas in order. The host sets every triangle up (snapped
-// centres, clipped bounding box, edges, attributes in rec words 4-6: u, v, the
-// vertex colours as packed BGR0 words, the vertex alphas in the w slots) and the
-// prefix sums of the boxes' pixels; the GPU rasterizes, sorts the fragments by
-// (pixel, triangle) and blends each pixel's fragments in order.
+// drawn into one canvas in order. The host clips every triangle's bounding box
+// and cuts it into work items; the GPU sets the triangles up, rasterizes and
+// shades their fragments into per-pixel lists and blends each list in triangle
+// order.
 struct DgOverlayJob {
-    const DgTriRec* rec;              // [n]
-    const uint4* box;                 // [n] (x_min, y_min, width, 0)
-    const unsigned long long* scan;   // [n + 1] exclusive prefix sums of the boxes' pixels
-    uint32_t n;
+    const float4* verts;              // [6 n] three vertices of (x, y, u, v, r, g, b, alpha) per triangle
+    const uint4* box;                 // [n] (x_min, y_min, width, pixels)
+    const uint2* items;               // [nitems] (triangle, first unit)
+    uint32_t n, nitems;
     uint32_t width, height;
     uint32_t* colour;                 // the canvas (BGRA, row 0 = top)
     const float* depth;               // y*W+x
     DgTexDev tex;                     // the RGBA map
-    uint64_t* fkey[2];                // fragment keys (pixel << 32 | triangle) and triangles
-    uint32_t* fval[2];
-    uint32_t fcap;
-    uint32_t* hist;
-    unsigned long long* cnt;          // [0] fragments emitted
+    uint4* node;                      // fragment nodes (as DgJobDev::fnode; key = the triangle)
+    uint32_t node_cap;                // every box pixel, and a partly used chunk per warp
+    uint32_t* head;                   // [width * height] list heads, kept zero between batches
+    unsigned long long* cnt;          // [0] nodes handed out, zero at the start
     uint32_t* err;
-    uint32_t sort_shift[8], n_sort;
+    uint32_t key_bits;                // bits of a triangle index
 };
+// Units (DG_UNIT_PX pixels) per work item of a box of npx pixels: four, and more
+// for boxes beyond a million pixels, so that one has at most 8192 items.
+constexpr uint32_t dg_overlay_units(uint64_t npx) {
+    const uint64_t per = (npx + DG_UNIT_PX * 8192ull - 1) / (DG_UNIT_PX * 8192ull);
+    return per < 4u ? 4u : (uint32_t)per;
+}
+#define DG_OVERLAY_BLOCKS_PER_SM 4u
+// blocks: the raster's grid (node_cap is sized for it).
 cudaError_t dg_launch_overlay(const DgOverlayJob& job, unsigned blocks, cudaStream_t s);
 // Scratch rows and records sized for a job of T triangles (shared sizing rule).
 constexpr uint64_t dg_trec_cap(uint64_t T) { return T + T / 8u + 4096u; }
