@@ -958,8 +958,11 @@ dg_status dg_ctx_destroy(dg_ctx* c) {
     slot_free(c->main);
     {
         OverlaySlot& O = c->overlay;
-        dfree(O.d_verts); dfree(O.d_box); dfree(O.d_items); dfree(O.d_node); dfree(O.d_head); dfree(O.d_cnt);
-        dfree(O.d_rgba);
+        dfree(O.d_in); dfree(O.d_node); dfree(O.d_head); dfree(O.d_rgba);
+        for (int k = 0; k < OverlaySlot::kStage; k++) {
+            if (O.h_stage[k]) cudaFreeHost(O.h_stage[k]);
+            if (O.stage_ev[k]) cudaEventDestroy(O.stage_ev[k]);
+        }
     }
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
@@ -1524,8 +1527,10 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
     if (e) return e;
     // host setup (canvas.rs:449-535): the bounding box of the snapped centres clipped
     // to the screen and the clipping rectangle, cut into work items
-    std::vector<uint4> box(n);
-    std::vector<uint2> items;
+    OverlaySlot& O = c->overlay;
+    std::vector<uint4>& box = O.box;
+    box.clear();
+    uint64_t nitems = 0;
     const HRect screen = HRect::from_coords(0, 0, cv->w - 1, cv->h - 1);
     unsigned long long total = 0;
     for (uint32_t t = 0; t < n; t++) {
@@ -1562,36 +1567,59 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
                 return DG_E_INVALID;
         }
         const uint64_t npx = (valid.w + 1) * (valid.h + 1);
-        box[t] = make_uint4((uint32_t)valid.x, (uint32_t)valid.y, (uint32_t)valid.w + 1u, (uint32_t)npx);
+        box.push_back(make_uint4((uint32_t)valid.x, (uint32_t)valid.y, (uint32_t)valid.w + 1u, (uint32_t)npx));
         total += npx;
-        if (total >= 0x7FFFFFFFull) continue;  // refused below
         const uint32_t units = (uint32_t)((npx + DG_UNIT_PX - 1) / DG_UNIT_PX), step = dg_overlay_units(npx);
-        for (uint32_t u = 0; u < units; u += step) items.push_back(make_uint2(t, u));
+        nitems += (units + step - 1) / step;
     }
     if (total >= 0x7FFFFFFFull) return DG_E_LIMIT;
     JobSlot& S = c->main;
-    OverlaySlot& O = c->overlay;
     const unsigned blocks = (unsigned)c->nsm * DG_OVERLAY_BLOCKS_PER_SM;
-    if ((e = grow(S, &O.d_verts, &O.verts_cap, 6ull * n)) || (e = grow(S, &O.d_box, &O.box_cap, n)) ||
-        (e = grow(S, &O.d_items, &O.items_cap, items.size())) ||
-        (e = grow(S, &O.d_node, &O.node_cap, dg_frag_nodes(total, blocks))) || (e = grow(S, &O.d_cnt, &O.cnt_cap, 1)))
+    const size_t o_verts = 16, o_box = o_verts + 96ull * n, o_items = o_box + 16ull * n, bytes = o_items + 8 * nitems;
+    if ((e = grow(S, &O.d_in, &O.in_cap, bytes)) ||
+        (e = grow(S, &O.d_node, &O.node_cap, dg_frag_nodes(total, blocks))))
         return e;
     if (O.head_cap < cv->w * cv->h) {
         if ((e = grow(S, &O.d_head, &O.head_cap, cv->w * cv->h))) return e;
         DG_CUDA(cudaMemsetAsync(O.d_head, 0, O.head_cap * sizeof(uint32_t), S.stream));
     }
-    DG_CUDA(cudaStreamSynchronize(S.stream));  // the scratch may still be read by the previous batch
-    DG_CUDA(cudaMemcpyAsync(O.d_verts, verts, n * 24ull * sizeof(float), cudaMemcpyHostToDevice, S.stream));
-    DG_CUDA(cudaMemcpyAsync(O.d_box, box.data(), n * sizeof(uint4), cudaMemcpyHostToDevice, S.stream));
-    DG_CUDA(cudaMemcpyAsync(O.d_items, items.data(), items.size() * sizeof(uint2), cudaMemcpyHostToDevice, S.stream));
-    DG_CUDA(cudaMemsetAsync(O.d_cnt, 0, sizeof(unsigned long long), S.stream));
+    const int k = O.stage;
+    O.stage = (O.stage + 1) % OverlaySlot::kStage;
+    if (!O.stage_ev[k])
+        DG_CUDA(cudaEventCreateWithFlags(&O.stage_ev[k], cudaEventDisableTiming));
+    else
+        DG_CUDA(cudaEventSynchronize(O.stage_ev[k]));  // this buffer's last upload has ended
+    if (O.stage_cap[k] < bytes) {
+        if (O.h_stage[k]) cudaFreeHost(O.h_stage[k]);
+        O.h_stage[k] = nullptr;
+        O.stage_cap[k] = 0;
+        const size_t cap = std::max<size_t>(bytes + bytes / 2, 64 * 1024);
+        if (cudaMallocHost(&O.h_stage[k], cap) != cudaSuccess) {
+            cudaGetLastError();
+            return DG_E_OOM;
+        }
+        O.stage_cap[k] = cap;
+    }
+    uint8_t* h = static_cast<uint8_t*>(O.h_stage[k]);
+    std::memset(h, 0, 16);
+    std::memcpy(h + o_verts, verts, 96ull * n);
+    std::memcpy(h + o_box, box.data(), 16ull * n);
+    uint2* items = reinterpret_cast<uint2*>(h + o_items);
+    for (uint32_t t = 0; t < n; t++) {
+        const uint32_t units = (box[t].w + DG_UNIT_PX - 1) / DG_UNIT_PX, step = dg_overlay_units(box[t].w);
+        for (uint32_t u = 0; u < units; u += step) *items++ = make_uint2(t, u);
+    }
+    // in stream order after the previous batch's kernels, which read the same device buffer
+    DG_CUDA(cudaMemcpyAsync(O.d_in, h, bytes, cudaMemcpyHostToDevice, S.stream));
+    DG_CUDA(cudaEventRecord(O.stage_ev[k], S.stream));
     DgOverlayJob j;
     std::memset(&j, 0, sizeof(j));
-    j.verts = O.d_verts;
-    j.box = O.d_box;
-    j.items = O.d_items;
+    j.cnt = reinterpret_cast<unsigned long long*>(O.d_in);
+    j.verts = reinterpret_cast<const float4*>(O.d_in + o_verts);
+    j.box = reinterpret_cast<const uint4*>(O.d_in + o_box);
+    j.items = reinterpret_cast<const uint2*>(O.d_in + o_items);
     j.n = n;
-    j.nitems = (uint32_t)items.size();
+    j.nitems = (uint32_t)nitems;
     j.width = (uint32_t)cv->w;
     j.height = (uint32_t)cv->h;
     j.colour = cv->d_colour;
@@ -1608,7 +1636,6 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
     j.node = O.d_node;
     j.node_cap = (uint32_t)std::min<size_t>(O.node_cap, 0xFFFFFFF0ull);
     j.head = O.d_head;
-    j.cnt = O.d_cnt;
     j.err = S.d_err;
     for (uint32_t b = n - 1; b; b >>= 1) j.key_bits++;
     DG_CUDA(dg_launch_overlay(j, blocks, S.stream));

@@ -197,18 +197,22 @@ struct JobSlot {
 namespace dgh {
 // Scratch of dg_canvas_draw_triangles_2d (grow-only, on the context stream).
 struct OverlaySlot {
-    float4* d_verts = nullptr;
-    size_t verts_cap = 0;
-    uint4* d_box = nullptr;
-    size_t box_cap = 0;
-    uint2* d_items = nullptr;
-    size_t items_cap = 0;
+    // One batch's upload: the node counter (16 bytes, zero), 96 bytes of vertices
+    // and 16 of box per triangle, 8 per work item. Built in a ring of pinned
+    // buffers, so a call neither waits for the frame before it nor stages its
+    // copies from pageable memory.
+    uint8_t* d_in = nullptr;
+    size_t in_cap = 0;
+    static const int kStage = 4;
+    void* h_stage[kStage] = {};
+    size_t stage_cap[kStage] = {};
+    cudaEvent_t stage_ev[kStage] = {};
+    int stage = 0;
+    std::vector<uint4> box;
     uint4* d_node = nullptr;
     size_t node_cap = 0;
     uint32_t* d_head = nullptr;  // zeroed at allocation; the fold clears what the raster sets
     size_t head_cap = 0;
-    unsigned long long* d_cnt = nullptr;
-    size_t cnt_cap = 0;
     uint32_t* d_rgba = nullptr;  // staging of dg_canvas_read_rgba
     size_t rgba_cap = 0;
 };
