@@ -436,13 +436,7 @@ dg_status sync_tex_table(dg_ctx* c, cudaStream_t stream) {
     std::vector<DgTexDev> t(c->tex.size());
     for (size_t i = 0; i < c->tex.size(); i++) {
         t[i].words = c->tex[i].d_words;
-        t[i].len = c->tex[i].len;
-        t[i].width = c->tex[i].w;
-        t[i].height = c->tex[i].h;
-        t[i].comps = c->tex[i].comps;
-        t[i].fw = (float)c->tex[i].w;
-        t[i].fh = (float)c->tex[i].h;
-        t[i].small = dg_tex_small(c->tex[i].len, c->tex[i].w, c->tex[i].h);
+        dg_tex_dims(t[i], c->tex[i].len, c->tex[i].w, c->tex[i].h, c->tex[i].comps);
         t[i].filter = c->tex[i].filter;
         t[i].pad = 0;
     }
@@ -1626,13 +1620,7 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
     j.depth = cv->d_depth;
     const TexMap& tm = c->tex[(size_t)(texmap + 1)];
     j.tex.words = tm.d_words;
-    j.tex.len = tm.len;
-    j.tex.width = tm.w;
-    j.tex.height = tm.h;
-    j.tex.comps = tm.comps;
-    j.tex.fw = (float)tm.w;
-    j.tex.fh = (float)tm.h;
-    j.tex.small = dg_tex_small(tm.len, tm.w, tm.h);
+    dg_tex_dims(j.tex, tm.len, tm.w, tm.h, tm.comps);
     j.node = O.d_node;
     j.node_cap = (uint32_t)std::min<size_t>(O.node_cap, 0xFFFFFFF0ull);
     j.head = O.d_head;

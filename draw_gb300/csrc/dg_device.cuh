@@ -64,9 +64,7 @@ __device__ __forceinline__ uint64_t as_usize(float f) {
     return (uint64_t)f;
 }
 __device__ __forceinline__ uint32_t as_u8(float f) {
-    if (!(f > 0.0f)) return 0u;
-    if (f >= 255.0f) return 255u;
-    return (uint32_t)f;
+    return min(__float2uint_rz(f), 255u);  // the conversion saturates, and NaN gives 0
 }
 
 // LLVM's powi lowering: binary exponentiation starting from r = 1 (r = 1*x is exact).
@@ -703,37 +701,38 @@ __device__ __forceinline__ void raster_box(const EdgeSet& e, float da, float db,
     }
 }
 
-// Texel fetch of TextureMap::get_rgb_slice (scene/mod.rs:154-168) with the
-// reference's wrapping usize arithmetic; false where the reference's slice
-// index would panic.
-__device__ __forceinline__ bool tex_rgb(const DgTexDev& tx, float u, float v, uint32_t& rgb) {
-    const float fu = floorf(fM(u, fS(tx.fw, 1.0f)));
-    const float fv = floorf(fM(v, fS(tx.fh, 1.0f)));
-    uint64_t off;
-    if (tx.small != 0u && fu >= 0.0f && fu < tx.fw && fv >= 0.0f && fv < tx.fh) {
-        // both indices inside the map: the wrapping usize arithmetic below reduces
-        // to this 32-bit one (the offset is below len < 2^32)
-        off = ((tx.height - 1u - (uint32_t)fv) * tx.width + (uint32_t)fu) * tx.comps;
-    } else {
-        const uint64_t ui = as_usize(fu);
-        const uint64_t vi = (uint64_t)tx.height - 1ull - as_usize(fv);
-        off = (vi * (uint64_t)tx.width + ui) * (uint64_t)tx.comps;
-    }
-    if (tx.len < 3ull || off > tx.len - 3ull) return false;
-    const uint64_t w = off >> 2;
-    const uint32_t sh = (uint32_t)(off & 3ull) * 8u;
-    const uint32_t lo = __ldg(tx.words + w);
-    // the three bytes span two words only when the offset is not word aligned
-    rgb = sh <= 8u ? (lo >> sh) : __funnelshift_r(lo, __ldg(tx.words + w + 1), sh);
-    return true;
-}
-
 // Three image bytes at byte offset off (off <= len - 3) as the low 24 bits.
 __device__ __forceinline__ uint32_t tex_bytes3(const DgTexDev& tx, uint64_t off) {
     const uint64_t w = off >> 2;
     const uint32_t sh = (uint32_t)(off & 3ull) * 8u;
     const uint32_t lo = __ldg(tx.words + w);
     return sh <= 8u ? (lo >> sh) : __funnelshift_r(lo, __ldg(tx.words + w + 1), sh);
+}
+
+// Texel fetch of TextureMap::get_rgb_slice (scene/mod.rs:154-168) with the
+// reference's wrapping usize arithmetic; false where the reference's slice
+// index would panic.
+__device__ __forceinline__ bool tex_rgb(const DgTexDev& tx, float u, float v, uint32_t& rgb) {
+    const float su = fM(u, tx.fw1), sv = fM(v, tx.fh1);
+    // floor and conversion in one: saturating, NaN -> 0, as floor and `as usize`
+    // give for indices inside the map
+    const uint32_t iu = (uint32_t)__float2int_rd(su), iv = (uint32_t)__float2int_rd(sv);
+    if (tx.small != 0u && iu < tx.width && iv < tx.height) {
+        // both indices inside the map: the wrapping usize arithmetic of the general
+        // path reduces to this 32-bit one (the offset is at most len - 3, len < 2^32)
+        const uint32_t off = ((tx.height - 1u - iv) * tx.width + iu) * tx.comps;
+        const uint32_t w = off >> 2, sh = (off & 3u) * 8u;
+        const uint32_t lo = __ldg(tx.words + w);
+        // the three bytes span two words only when the offset is not word aligned
+        rgb = sh <= 8u ? (lo >> sh) : __funnelshift_r(lo, __ldg(tx.words + w + 1u), sh);
+        return true;
+    }
+    const uint64_t ui = as_usize(floorf(su));
+    const uint64_t vi = (uint64_t)tx.height - 1ull - as_usize(floorf(sv));
+    const uint64_t off = (vi * (uint64_t)tx.width + ui) * (uint64_t)tx.comps;
+    if (tx.len < 3ull || off > tx.len - 3ull) return false;
+    rgb = tex_bytes3(tx, off);
+    return true;
 }
 
 // Extension (no counterpart in the reference, which samples the nearest texel):
@@ -745,7 +744,7 @@ __device__ __forceinline__ uint32_t tex_bytes3(const DgTexDev& tx, uint64_t off)
 // t0 = c00 (1 - ax) + c01 ax, t1 = c10 (1 - ax) + c11 ax, c = t0 (1 - ay) + t1 ay.
 // False (the texture-range error) when any of the four offsets is past the image.
 __device__ __noinline__ bool tex_bilinear(const DgTexDev& tx, float u, float v, const float* inv255, V3& out) {
-    const float x = fM(u, fS(tx.fw, 1.0f)), y = fM(v, fS(tx.fh, 1.0f));
+    const float x = fM(u, tx.fw1), y = fM(v, tx.fh1);
     const float fx = floorf(x), fy = floorf(y);
     const float ax = fS(x, fx), ay = fS(y, fy);
     const uint64_t ui = as_usize(fx);
@@ -836,20 +835,29 @@ __device__ __forceinline__ uint32_t shade_colour(const DgJobDev& job, const DgTe
     V3 inner = c_a;
 #pragma unroll
     for (uint32_t l = 0; l < DG_MAXL; l++) {
-        if (l < nl) {
-            V3 lt, h;
-            lv(l, lt, h);
-            const float ln = vdot(lt, pn);
-            const float mx = ln > 0.0f ? ln : 0.0f;  // 0.0_f32.max(x): NaN -> 0
-            inner = vadd(inner, vmul(c_l, fS(1.0f, mx)));
-            hn[l] = vdot(h, pn);
-        }
+        if (l >= nl) break;
+        V3 lt, h;
+        lv(l, lt, h);
+        const float ln = vdot(lt, pn);
+        const float mx = ln > 0.0f ? ln : 0.0f;  // 0.0_f32.max(x): NaN -> 0
+        inner = vadd(inner, vmul(c_l, fS(1.0f, mx)));
+        hn[l] = vdot(h, pn);
     }
     V3 col = {fM(c_r.x, inner.x), fM(c_r.y, inner.y), fM(c_r.z, inner.z)};
     const int32_t ex = fr.exponent;
+    if (ex == 2) {  // the reference's exponent: powi(x, 2) is x * x
 #pragma unroll
-    for (uint32_t l = 0; l < DG_MAXL; l++)
-        if (l < nl) col = vadd(col, vmul(c_l, powi(hn[l], ex)));
+        for (uint32_t l = 0; l < DG_MAXL; l++) {
+            if (l >= nl) break;
+            col = vadd(col, vmul(c_l, fM(hn[l], hn[l])));
+        }
+    } else {
+#pragma unroll
+        for (uint32_t l = 0; l < DG_MAXL; l++) {
+            if (l >= nl) break;
+            col = vadd(col, vmul(c_l, powi(hn[l], ex)));
+        }
+    }
     // Pixel::from_normalized_vec3 (canvas.rs:89-92), stored as b,g,r,255
     const V3 sc = vmul(col, 255.0f);
     const uint32_t R = as_u8(sc.x), G = as_u8(sc.y), B = as_u8(sc.z);
@@ -858,7 +866,8 @@ __device__ __forceinline__ uint32_t shade_colour(const DgJobDev& job, const DgTe
 
 // Row `row` of the light/halfway table for light l: (lt.x, lt.y, lt.z, h.x), (h.y, h.z, -, -).
 __device__ __forceinline__ const float4* shade_row(const DgJobDev& job, uint32_t row, uint32_t l) {
-    return job.vshade + ((uint64_t)row * job.shade_stride + l) * 2;
+    // the row's address first (one widening multiply), so that the lights are immediate offsets
+    return job.vshade + (uint64_t)row * (job.shade_stride * 2u) + l * 2u;
 }
 
 // Shades the winning fragment of pixel (x, y) from its triangle record:

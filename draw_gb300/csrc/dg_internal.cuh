@@ -79,10 +79,10 @@ __device__ __forceinline__ bool dg_check_range(bool ok, uint32_t* err) {
 // so kernels read them with 16-byte loads.
 struct alignas(16) DgTexDev {
     const uint32_t* words;  // image bytes, little-endian in u32 words, one pad word at the end
-    uint64_t len;           // image length in bytes
+    float fw1, fh1;         // width as f32, less 1.0; height as f32, less 1.0
     uint32_t width, height, comps;
-    float fw, fh;           // width as f32, height as f32
-    uint32_t small;         // 1 if len < 2^32 and width, height < 2^24 (32-bit texel offsets suffice)
+    uint32_t small;         // dg_tex_small: the nearest fetch's short path
+    uint64_t len;           // image length in bytes
     uint32_t filter;        // DG_FILTER_NEAREST (the reference) or DG_FILTER_BILINEAR (extension)
     uint32_t pad;
 };
@@ -128,8 +128,19 @@ struct alignas(16) DgFrameDev {
 // (DG_TRI_LAZY in the record's tie word).
 #define DG_FRAME_LAZY 2u
 static_assert(sizeof(DgTexDev) == 48 && sizeof(DgMatDev) == 48, "descriptor sizes");
-inline uint32_t dg_tex_small(uint64_t len, uint64_t w, uint64_t h) {
-    return (len < (1ull << 32) && w < (1ull << 24) && h < (1ull << 24)) ? 1u : 0u;
+// 1 if texel indices inside the map need neither 64-bit offsets nor a check of
+// the three bytes against len (len = width * height * comps).
+inline uint32_t dg_tex_small(uint64_t len, uint64_t w, uint64_t h, uint64_t comps) {
+    return (len < (1ull << 32) && w < (1ull << 24) && h < (1ull << 24) && comps >= 3) ? 1u : 0u;
+}
+inline void dg_tex_dims(DgTexDev& t, uint64_t len, uint32_t w, uint32_t h, uint32_t comps) {
+    t.len = len;
+    t.width = w;
+    t.height = h;
+    t.comps = comps;
+    t.fw1 = (float)w - 1.0f;
+    t.fh1 = (float)h - 1.0f;
+    t.small = dg_tex_small(len, w, h, comps);
 }
 static_assert(sizeof(DgFrameDev) % 16 == 0, "frame descriptor size");
 // 16-byte words of DgFrameDev read with vector loads by the kernels.

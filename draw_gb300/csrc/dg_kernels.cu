@@ -850,33 +850,39 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const uint
 #pragma unroll
     for (int j = 0; j < R; j++) {  // all loads first: R keys in flight per thread
         const uint32_t y = ty * TH + wid + 8u * j;
-        key[j] = (x < W && y < H) ? __ldcg(reinterpret_cast<const unsigned long long*>(fr.vis) + (uint64_t)y * W + x)
+        key[j] = (x < W && y < H) ? __ldcg(reinterpret_cast<const unsigned long long*>(fr.vis) + (y * W + x))
                                   : DG_VIS_EMPTY - 1ull;  // outside the canvas
     }
+    const bool one_seg = fr.seg_count == 1u;
+    const DgSegDev& sg0 = job.segs[one_seg ? fr.seg_begin : 0u];
+    const uint32_t* rec0 = job.rec_of + sg0.tri_begin;
+    const uint32_t ntri0 = sg0.ntri;
     uint32_t val[R];
     unsigned hit[R];
     int no_record = 0;
 #pragma unroll
     for (int j = 0; j < R; j++) {
         const uint32_t y = ty * TH + wid + 8u * j;
-        const uint64_t i = (uint64_t)y * W + x;
-        const bool covered_px = key[j] < DG_VIS_EMPTY - 1ull;
+        const uint32_t i = y * W + x;  // below 2^31 (pixels of a job)
         val[j] = DG_NONE;
         if (key[j] == DG_VIS_EMPTY) {
             fr.depth[i] = fr.clear_depth;
-            fr.colour[(uint64_t)(H - 1u - y) * W + x] = AZUL_BB;
-        } else if (covered_px) {
+            fr.colour[(H - 1u - y) * W + x] = AZUL_BB;
+        } else if (key[j] != DG_VIS_EMPTY - 1ull) {
             // the triangle record of the key: segment of the submission index, then rec_of
-            const uint32_t seq = (uint32_t)key[j];
-            const uint32_t tl = seq >> 2;
-            const uint32_t si = fr.seg_begin + last_le(fr.seg_count, tl, [&](uint32_t k) {
-                                    return job.segs[fr.seg_begin + k].seq_base;
-                                });
-            const DgSegDev& sg = job.segs[si];
-            const uint32_t t = tl - sg.seq_base;
-            if (t < sg.ntri) val[j] = __ldg(job.rec_of + sg.tri_begin + t);
+            const uint32_t tl = (uint32_t)key[j] >> 2;
+            if (one_seg) {
+                if (tl < ntri0) val[j] = __ldg(rec0 + tl);
+            } else {
+                const uint32_t si = fr.seg_begin + last_le(fr.seg_count, tl, [&](uint32_t k) {
+                                        return job.segs[fr.seg_begin + k].seq_base;
+                                    });
+                const DgSegDev& sg = job.segs[si];
+                const uint32_t t = tl - sg.seq_base;
+                if (t < sg.ntri) val[j] = __ldg(job.rec_of + sg.tri_begin + t);
+            }
             const uint32_t o = (uint32_t)key[j] & 3u;
-            if (val[j] != DG_NONE && (uint64_t)val[j] + o < job.trec_cap) {
+            if (val[j] != DG_NONE && val[j] + o < job.trec_cap) {  // trec_cap <= 2^32 - 16
                 val[j] += o;
                 fr.vis[i] = DG_VIS_EMPTY;
             } else {
@@ -884,7 +890,7 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const uint
                 no_record = 1;
             }
         }
-        hit[j] = __ballot_sync(FULL, covered_px && val[j] != DG_NONE);
+        hit[j] = __ballot_sync(FULL, val[j] != DG_NONE);
         if (lane == 0) s_row[wid + 8u * j] = __popc(hit[j]);
     }
     const int any_no_record = __syncthreads_or(no_record);
@@ -914,6 +920,7 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const uint
     }
     __syncthreads();
     const uint32_t n = s_row[32];
+    uint32_t errors = 0;
     for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
         const uint32_t pe = s_pix[k];
         const uint32_t px = tx * DG_TILE_W + (pe & 31u), py = ty * TH + (pe >> 5);
@@ -921,14 +928,16 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const uint
         int errc;
         const float4* wp = EXT && (fr.flags & DG_FRAME_PERSPECTIVE) && job.trec_w ? job.trec_w + s_val[k] : nullptr;
         uint32_t c = shade_from_record<EXT, LAZY>(job, fr, job.trec + s_val[k], px, py, inv255, stex, d, errc, wp);
-        if (errc != DG_OK) c = AZUL_BB;
-        // one error-word update per warp (every pixel of a bad job may fail)
-        const unsigned act = __activemask();
-        const uint32_t bits = __reduce_or_sync(act, errc != DG_OK ? 1u << errc : 0u);
-        if (bits != 0u && lane == (uint32_t)(__ffs(act) - 1)) atomicOr(job.err, bits);
-        fr.depth[(uint64_t)py * W + px] = d;
-        fr.colour[(uint64_t)(H - 1u - py) * W + px] = c;
+        if (errc != DG_OK) {
+            c = AZUL_BB;
+            errors |= 1u << errc;
+        }
+        fr.depth[py * W + px] = d;
+        fr.colour[(H - 1u - py) * W + px] = c;
     }
+    // one error-word update per warp (every pixel of a bad job may fail)
+    errors = __reduce_or_sync(FULL, errors);
+    if (errors != 0u && lane == 0u) atomicOr(job.err, errors);
     // pixels whose triangle has no record: shaded the long way (block-uniform)
     if (any_no_record) shade_tile_without_records<TH>(job, tile, inv255, stex);
 }

@@ -189,20 +189,10 @@ extern "C" dg_status dg_render_noalloc(const dg_frame_params* p, const dg_device
 
     // texture table: [0] the 1x1 white default map (scene/mod.rs:128-135), then the caller's maps
     d.tex[0].words = reinterpret_cast<const uint32_t*>(base + kOffWhite);
-    d.tex[0].len = 3;
-    d.tex[0].width = d.tex[0].height = 1;
-    d.tex[0].comps = 3;
-    d.tex[0].fw = d.tex[0].fh = 1.0f;
-    d.tex[0].small = 1;
+    dg_tex_dims(d.tex[0], 3, 1, 1, 3);
     for (uint32_t i = 0; i < ntex; i++) {
         d.tex[i + 1].words = static_cast<const uint32_t*>(texmaps[i].bytes);
-        d.tex[i + 1].len = texmaps[i].len;
-        d.tex[i + 1].width = texmaps[i].width;
-        d.tex[i + 1].height = texmaps[i].height;
-        d.tex[i + 1].comps = texmaps[i].components;
-        d.tex[i + 1].fw = (float)texmaps[i].width;
-        d.tex[i + 1].fh = (float)texmaps[i].height;
-        d.tex[i + 1].small = dg_tex_small(texmaps[i].len, texmaps[i].width, texmaps[i].height);
+        dg_tex_dims(d.tex[i + 1], texmaps[i].len, texmaps[i].width, texmaps[i].height, texmaps[i].components);
     }
     for (uint32_t i = 0; i < nmat; i++) {
         for (int k = 0; k < 3; k++) {

@@ -678,8 +678,8 @@ __global__ void __launch_bounds__(256) k_tfold(const __grid_constant__ DgJobDev 
 // (v * height) floored, wrapping usize offset, four bytes; false where the
 // reference's slice index would panic.
 __device__ __forceinline__ bool tex_rgba(const DgTexDev& tx, float u, float v, uint32_t& rgba) {
-    const uint64_t ui = as_usize(floorf(fM(u, tx.fw)));
-    const uint64_t vi = (uint64_t)tx.height - 1ull - as_usize(floorf(fM(v, tx.fh)));
+    const uint64_t ui = as_usize(floorf(fM(u, (float)tx.width)));
+    const uint64_t vi = (uint64_t)tx.height - 1ull - as_usize(floorf(fM(v, (float)tx.height)));
     const uint64_t off = (vi * (uint64_t)tx.width + ui) * (uint64_t)tx.comps;
     if (tx.len < 4ull || off > tx.len - 4ull) return false;
     const uint64_t w = off >> 2;
