@@ -211,19 +211,47 @@ __device__ __forceinline__ void make_edges(float ax, float ay, float bx, float b
         fast = fast && e.den[k] > 0.0f && e.den[k] < INFINITY;
     }
     if (fast) e.tie |= DG_EDGE_FAST;
+    // div_rcp: every den is finite, > 0 and below 2^100 (DG_EDGE_FAST makes them
+    // integer-valued and so >= 1), |A|, |B| < 2^64 and |C|, |D| < 2^98, so that the
+    // edge value at any pixel (coordinates below 2^32) stays below 2^100 in magnitude.
+    bool rcp = fast, span = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float ab = fmaxf(fabsf(e.A[k]), fabsf(e.B[k])), cd = fmaxf(fabsf(e.C[k]), fabsf(e.D[k]));
+        rcp = rcp && e.den[k] < 0x1p100f && ab < 0x1p64f && cd < 0x1p98f;
+        span = span && ab < 0x1p24f && cd < 0x1p30f;
+    }
+    if (rcp) e.tie |= DG_EDGE_RCP | (span ? DG_EDGE_SPAN : 0u);
 }
 
-// Whether the barycentric divisions of an edge set may use div_rcp: every den
-// is finite, > 0 and below 2^100 (DG_EDGE_FAST makes them integer-valued and so
-// >= 1), |A|, |B| < 2^64 and |C|, |D| < 2^98, so that the edge value at any
-// pixel (coordinates below 2^32) stays below 2^100 in magnitude.
-__device__ __forceinline__ bool edge_rcp_ok(const EdgeSet& e) {
-    bool ok = (e.tie & DG_EDGE_FAST) != 0u;
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-        ok = ok && e.den[k] < 0x1p100f && fabsf(e.A[k]) < 0x1p64f && fabsf(e.B[k]) < 0x1p64f &&
-             fabsf(e.C[k]) < 0x1p98f && fabsf(e.D[k]) < 0x1p98f;
-    return ok;
+// Narrows [lo, hi] to the pixels x of row y at which edge k passes the coverage
+// test of DG_EDGE_FAST triangles (its value > 0, or 0 with the tie bit). Every
+// rounded operation of the edge value is monotone in x, so these pixels are one
+// side of the row; the boundary is estimated from rA (about 1/A) and then moved
+// by the exact test itself, so the result does not depend on the estimate.
+// Called for DG_EDGE_SPAN edge sets (finite values, an estimate within a few
+// pixels); [x0, x1] is the row's range, hi < lo an empty result.
+__device__ __forceinline__ void row_span(const EdgeSet& e, int k, float rA, float yf, int x0, int x1, int& lo, int& hi) {
+    const float by = fM(e.B[k], yf);
+    const bool tie = (e.tie >> k) & 1u;
+    auto in = [&](int x) {
+        const float f = fS(fA(fA(fM(e.A[k], (float)x), by), e.C[k]), e.D[k]);
+        return f > 0.0f || (f == 0.0f && tie);
+    };
+    const float est = ((e.D[k] - e.C[k]) - by) * rA;
+    if (e.A[k] > 0.0f) {  // from the boundary to the right
+        int x = (int)fminf(fmaxf(ceilf(est), (float)x0), (float)(x1 + 1));
+        while (x > x0 && in(x - 1)) x--;
+        while (x <= x1 && !in(x)) x++;
+        lo = max(lo, x);
+    } else if (e.A[k] < 0.0f) {  // up to the boundary
+        int x = (int)fminf(fmaxf(floorf(est), (float)(x0 - 1)), (float)x1);
+        while (x < x1 && in(x + 1)) x++;
+        while (x >= x0 && !in(x)) x--;
+        hi = min(hi, x);
+    } else if (!in(x0)) {  // the same value along the row
+        hi = x0 - 1;
+    }
 }
 
 // Division-free early reject, exact with respect to the reference's test.
@@ -661,7 +689,7 @@ __device__ __forceinline__ void raster_box(const EdgeSet& e, float da, float db,
             }
         }
         if (!mask) return;
-        const bool rcp = edge_rcp_ok(e);
+        const bool rcp = (e.tie & DG_EDGE_RCP) != 0u;
         const float y0 = rcp ? __frcp_rn(e.den[0]) : 0.0f, y1 = rcp ? __frcp_rn(e.den[1]) : 0.0f,
                     y2 = rcp ? __frcp_rn(e.den[2]) : 0.0f;
         // k / w for k < 64 and w <= 64: k * ceil(2^16 / w) >> 16 errs by less than

@@ -54,10 +54,9 @@ __device__ __forceinline__ bool dg_check_range(bool ok, uint32_t* err) {
 
 // Triangles whose clipped bounding box has at most DgFrameDev.small_max_px
 // pixels go to the small-triangle list, whose entries the queue pass
-// rasterizes one per lane; larger ones go to the raster queue: their row-major
-// bounding-box pixels are cut into units of DG_UNIT_PX (one per lane of a warp)
-// and the units into work items of at most DgJobDev.item_units (default
-// DG_ITEM_UNITS), which the queue pass spreads over all warps. Unless the
+// rasterizes one per lane; larger ones go to the raster queue: their bounding
+// box is cut into work items (DgItemGrid) of about 128 * DgJobDev.item_units
+// pixels (default DG_ITEM_UNITS), which the queue pass spreads over all warps. Unless the
 // tuning fixes it, a frame's threshold is DG_SMALL_MAX_PX, or
 // DG_SMALL_MAX_PX_MICRO when the frame has at least as many triangles as
 // pixels: lanes that each loop over a box of up to 64 pixels pay off only when
@@ -184,12 +183,17 @@ struct DgSegDev {
 struct DgEdges {
     float A[3], B[3], C[3], D[3];
     float den[3];  // f_alpha = f_bc(a), f_beta = f_ca(b), f_gama = f_ab(c)
-    uint32_t tie;  // bit k: den[k] * f_k(-1, -1) > 0 (the reference's tie rule); DG_EDGE_FAST
+    uint32_t tie;  // bit k: den[k] * f_k(-1, -1) > 0 (the reference's tie rule); DG_EDGE_* flags
 };
 
 // Set in DgEdges.tie when every den is finite and > 0 (edges are stored
 // normalized to a den without sign bit): coverage is then a sign test.
 #define DG_EDGE_FAST 8u
+// Set in DgEdges.tie when the barycentric divisions may use div_rcp
+// (dg_device.cuh), and when moreover the edge constants are small enough that a
+// row's covered span can be estimated to within a few pixels (row_span).
+#define DG_EDGE_RCP 32u
+#define DG_EDGE_SPAN 64u
 // Set in a triangle record's tie word when its vertices have no light/halfway
 // rows (DG_FRAME_LAZY): shading computes them from the vertex positions, with
 // the same functions that fill the rows, so the values are identical.
@@ -214,19 +218,38 @@ struct alignas(16) DgTriRec {
 };
 static_assert(sizeof(DgTriRec) == 192, "triangle record size");
 
-// A triangle queued for the load-balanced raster pass (32 bytes). Its clipped
-// bounding box's pixels, numbered row-major, are cut into units of DG_UNIT_PX
-// consecutive pixels, one per lane. Entries of the small-triangle list use the
-// same layout with npx holding the box height and nunits unused.
+// A triangle queued for the load-balanced raster pass, or an entry of the
+// small-triangle list (32 bytes).
 struct alignas(16) DgQueueRec {
     uint32_t rec;     // its DgTriRec
     uint32_t seq;     // frame-local key low word
     uint32_t frame;
     uint32_t xlo, ylo;  // clipped bounding box origin
-    uint32_t w;         // bounding box width in pixels
-    uint32_t npx;       // bounding box pixels
-    uint32_t nunits;    // ceil(npx / DG_UNIT_PX)
+    uint32_t w, h;      // bounding box size in pixels
+    uint32_t pad;
 };
+
+// How the box of a queued triangle is cut into work items: a grid of nx columns
+// of items, each cw x rh pixels (the last ones less). A warp finds the covered
+// span of up to 32 rows at once, so an item is 32 rows high and as wide as
+// keeps it at about 128 * item_units pixels, wider for boxes of fewer rows and
+// several times 32 rows high for boxes of fewer columns.
+struct DgItemGrid {
+    uint32_t cw, rh, nx, n;
+};
+__host__ __device__ inline DgItemGrid dg_item_grid(uint32_t w, uint32_t h, uint32_t item_units) {
+    const uint32_t px = 128u * item_units;
+    uint32_t pw = 1u, ph = 1u;  // box size rounded up to a power of two, at most 32
+    while (pw < w && pw < 32u) pw *= 2u;
+    while (ph < h && ph < 32u) ph *= 2u;
+    DgItemGrid g;
+    g.cw = w <= 32u ? w : px / ph;  // at least 4
+    const uint32_t rows = (px / pw) & ~31u;
+    g.rh = w <= 32u && rows > 32u ? rows : 32u;
+    g.nx = (w + g.cw - 1u) / g.cw;
+    g.n = g.nx * ((h + g.rh - 1u) / g.rh);
+    return g;
+}
 
 #define DG_NONE 0xFFFFFFFFu
 // Job counters (unsigned long long each), each on its own 128-byte line: the
@@ -273,11 +296,11 @@ struct DgJobDev {
     uint32_t trec_cap;
     uint32_t queue_cap;
     DgQueueRec* queue;
-    uint2* items;           // work items: (queue record, first unit)
+    uint2* items;           // work items: (queue record, number in its grid)
     uint32_t items_cap;
-    DgQueueRec* small;      // small-triangle list (nunits unused), rasterized one triangle per lane
+    DgQueueRec* small;      // small-triangle list, rasterized one triangle per lane
     uint32_t small_cap;
-    uint32_t item_units;    // work units per raster work item (>= 1)
+    uint32_t item_units;    // size of the raster work items in 128 pixels (>= 1)
     uint32_t total_px;      // pixels of all frames
     uint32_t tile_rows;     // resolve tile height (8, 16 or 32)
     unsigned long long* cnt;  // the job counters (DG_CNT_*, DG_NCOUNTERS words), zero at the start of the job

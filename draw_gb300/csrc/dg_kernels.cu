@@ -307,8 +307,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 RTri tr;
                 EdgeSet e;
                 bool small = false;  // goes to the small-triangle list
-                uint32_t nu = 0;     // work units to queue (0: not queued)
-                uint32_t qpx = 0;    // bounding-box pixels of the queued triangle
+                uint32_t nu = 0;     // 32-pixel units of the box to queue (0: not queued)
                 bool inplace = false;
                 bool boxed = false;  // the triangle has a box (no NaN centre)
                 tr.xlo = tr.xhi = tr.ylo = tr.yhi = 0;
@@ -357,7 +356,6 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                         } else if (px <= fr.small_max_px) {
                             small = true;
                         } else {
-                            qpx = (uint32_t)px;  // below 2^31: the canvas has fewer pixels
                             nu = (uint32_t)((px + DG_UNIT_PX - 1u) / DG_UNIT_PX);
                         }
                     }
@@ -401,7 +399,8 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 // items, each lane taking every 32nd.
                 const unsigned qmask = __ballot_sync(FULL, nu != 0u);
                 if (qmask) {
-                    const uint32_t ni = (nu + job.item_units - 1u) / job.item_units;
+                    const uint32_t bw = tr.xhi - tr.xlo + 1u, bh = tr.yhi - tr.ylo + 1u;
+                    const uint32_t ni = nu ? dg_item_grid(bw, bh, job.item_units).n : 0u;
                     uint32_t incl = ni, uincl = nu;
     #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
@@ -428,7 +427,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                     if (fits) {
                         uint4* qd = reinterpret_cast<uint4*>(job.queue + rec);
                         qd[0] = make_uint4(rbase + (uint32_t)rr, tr.seq, tr.frame, tr.xlo);
-                        qd[1] = make_uint4(tr.ylo, tr.xhi - tr.xlo + 1u, qpx, nu);
+                        qd[1] = make_uint4(tr.ylo, bw, bh, 0u);
                     } else if (nu != 0u) {
                         inplace = true;  // queue full: this lane rasterizes the box itself
                     }
@@ -444,7 +443,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                         const bool ofits = __shfl_sync(FULL, fits ? 1u : 0u, L) != 0u;
                         for (uint32_t k = lane; k < lni; k += 32u)
                             if (oib + k < job.items_cap)
-                                job.items[oib + k] = ofits ? make_uint2(orec, k * job.item_units) : make_uint2(DG_NONE, 0u);
+                                job.items[oib + k] = ofits ? make_uint2(orec, k) : make_uint2(DG_NONE, 0u);
                     }
                     // The other lanes' items numbered together: item j belongs to the first lane
                     // whose inclusive count exceeds it.
@@ -474,7 +473,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                         const bool ofits = __shfl_sync(FULL, fits ? 1u : 0u, lo) != 0u;
                         const uint32_t k = j - oex;  // item index within its record
                         if (j < stotal && oib + k < job.items_cap)
-                            job.items[oib + k] = ofits ? make_uint2(orec, k * job.item_units) : make_uint2(DG_NONE, 0u);
+                            job.items[oib + k] = ofits ? make_uint2(orec, k) : make_uint2(DG_NONE, 0u);
                     }
                 }
                 // Small triangles go to the small-triangle list (one atomic per warp), which the
@@ -515,53 +514,10 @@ __global__ void __launch_bounds__(256) k_setup_raster(const DgJobDev job) {
     dev_setup(job);
 }
 
-// The raster queue: the bounding-box pixels of every queued triangle in
-// row-major units of DG_UNIT_PX (one pixel per lane), grouped into work items
-// of at most job.item_units units that the warps take in a strided order.
-// One candidate fragment of a queued triangle (its pixel passed prereject):
-// the coverage test with the divisions, the depth, the strict test against the
-// clear depth and the keyed minimum.
-// rcp (uniform over the warp): the edge set passed edge_rcp_ok and yr holds the
-// reciprocals of its three dens.
-// The edge set and the vertex depths are read from the record R (cached: every
-// call of a work item reads the same words), which keeps them out of the unit
-// loop's registers.
-__device__ __forceinline__ void finish_fragment(const DgTriRec* R, uint32_t seq, uint32_t x, uint32_t y,
-                                                float clear_depth, unsigned long long* vis, uint32_t width, bool rcp,
-                                                float3 yr) {
-    EdgeSet e;
-    load_edges(R, e);
-    const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
-    float al, be, ga;
-    const float xf = (float)x, yf = (float)y;
-    const float n0 = edge_eval(e, 0, xf, yf), n1 = edge_eval(e, 1, xf, yf), n2 = edge_eval(e, 2, xf, yf);
-    bool cov;
-    if (rcp) {  // the candidate passed the sign test: only the barycentrics remain
-        al = div_rcp(n0, e.den[0], yr.x);
-        be = div_rcp(n1, e.den[1], yr.y);
-        ga = div_rcp(n2, e.den[2], yr.z);
-        cov = true;
-    } else if (e.tie & DG_EDGE_FAST) {
-        al = fD(n0, e.den[0]);
-        be = fD(n1, e.den[1]);
-        ga = fD(n2, e.den[2]);
-        cov = true;
-    } else {
-        cov = covered_divide(e, n0, n1, n2, al, be, ga);
-    }
-    if (cov) {
-        const float depth = interp(al, be, ga, dd.x, dd.y, dd.z);
-        if (depth < clear_depth) atomicMin(vis + (uint64_t)y * width + x, depth_key(depth, seq));
-    }
-}
-
 __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
-    __shared__ uint32_t s_bx[8][64], s_by[8][64];  // per-warp candidate buffers
     __shared__ uint32_t s_sorted[256];             // a group of small triangles in box-size order
     __shared__ uint32_t s_bucket[16];              // their counts, then offsets, per box-size class
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t* bx = s_bx[threadIdx.x >> 5];
-    uint32_t* by = s_by[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     // Prologue: light/halfway vectors of the vertices the setup pass marked, 32
@@ -646,73 +602,69 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
         const DgTriRec* R = job.trec + q0.x;
         EdgeSet e;
         load_edges(R, e);
+        const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
         const uint32_t seq = q0.y;
         const DgFrameDev& fr = job.frames[q0.z];
         const float clear_depth = fr.clear_depth;
         unsigned long long* vis = reinterpret_cast<unsigned long long*>(fr.vis);
         const uint32_t width = fr.width;
-        const uint32_t xlo = q0.w, ylo = q1.x, w = q1.y, npx = q1.z;
-        if (!DG_IN_RANGE(w != 0u && xlo + w <= width && ylo + (npx + w - 1u) / w <= fr.height && q0.x < job.trec_cap,
-                         job.err))
+        const uint32_t xlo = q0.w, ylo = q1.x, w = q1.y, h = q1.z;
+        if (!DG_IN_RANGE(w != 0u && xlo + w <= width && ylo + h <= fr.height && q0.x < job.trec_cap, job.err)) continue;
+        const DgItemGrid grid = dg_item_grid(w, h, job.item_units);
+        const uint32_t iy = grid.nx == 1u ? item.y : item.y / grid.nx, ix = item.y - iy * grid.nx;
+        const uint32_t x0 = xlo + ix * grid.cw, xe = min(x0 + grid.cw, xlo + w);  // columns [x0, xe)
+        const uint32_t y0 = ylo + iy * grid.rh, ye = min(y0 + grid.rh, ylo + h);  // rows [y0, ye)
+        if (!(e.tie & DG_EDGE_SPAN)) {  // huge or not finite edge constants: the reference's test per pixel
+            const uint32_t cw = xe - x0, n = cw * (ye - y0);
+            for (uint32_t k = lane; k < n; k += 32u) raster_pixel(e, dd.x, dd.y, dd.z, seq, x0 + k % cw, y0 + k / cw, fr);
+            __syncwarp();
             continue;
-        const uint32_t u_end = min(q1.w, item.y + job.item_units);
-        // Stage A: every lane takes one pixel of the unit and applies the exact,
-        // division-free pre-reject; candidates are packed into the warp's buffer.
-        // Stage B: whenever 32 candidates are buffered, each lane finishes one of
-        // them (the reference's full test with its three divisions, then the
-        // depth key), so the division path runs with all lanes busy.
-        uint32_t pending = 0;
-        const bool fast = (e.tie & DG_EDGE_FAST) != 0u;
-        const bool rcp = edge_rcp_ok(e);
-        const float3 yr = rcp ? make_float3(__frcp_rn(e.den[0]), __frcp_rn(e.den[1]), __frcp_rn(e.den[2]))
-                              : make_float3(0.0f, 0.0f, 0.0f);
-        // This lane's pixel k = u * DG_UNIT_PX + lane of the box, as column xx and
-        // row yy: one division per item, then a step of DG_UNIT_PX pixels per unit
-        // (q32 rows and r32 columns, with at most one carry since xx, r32 < w).
-        uint32_t k = item.y * DG_UNIT_PX + lane;
-        uint32_t yy = k / w, xx = k - yy * w;
-        const uint32_t q32 = DG_UNIT_PX / w, r32 = DG_UNIT_PX - q32 * w;
-        // Buffers this unit's candidates and finishes 32 whenever that many are buffered.
-        auto push = [&](bool cand, uint32_t x, uint32_t y) {
-            const unsigned b = __ballot_sync(FULL, cand);
-            if (cand) {
-                const uint32_t slot = pending + __popc(b & ((1u << lane) - 1u));
-                bx[slot] = x;
-                by[slot] = y;
-            }
-            pending += __popc(b);
-            if (pending >= 32u) {
-                __syncwarp();
-                finish_fragment(R, seq, bx[lane], by[lane], clear_depth, vis, width, rcp, yr);
-                __syncwarp();
-                if (lane < pending - 32u) {
-                    bx[lane] = bx[32u + lane];
-                    by[lane] = by[32u + lane];
-                }
-                __syncwarp();
-                pending -= 32u;
-            }
-        };
-        for (uint32_t u = item.y; u < u_end; u++, k += DG_UNIT_PX) {
-            bool cand = false;
-            const uint32_t x = xlo + xx, y = ylo + yy;
-            xx += r32;
-            yy += q32;
-            if (xx >= w) {
-                xx -= w;
-                yy++;
-            }
-            if (k < npx) {
-                const float xf = (float)x, yf = (float)y;
-                const float n0 = edge_eval(e, 0, xf, yf), n1 = edge_eval(e, 1, xf, yf), n2 = edge_eval(e, 2, xf, yf);
-                cand = fast ? covered_signs(e.tie, n0, n1, n2)
-                            : !(prereject(n0, e.den[0]) || prereject(n1, e.den[1]) || prereject(n2, e.den[2]));
-            }
-            push(cand, x, y);
         }
-        __syncwarp();
-        if (lane < pending) finish_fragment(R, seq, bx[lane], by[lane], clear_depth, vis, width, rcp, yr);
-        __syncwarp();
+        const float3 yr = make_float3(__frcp_rn(e.den[0]), __frcp_rn(e.den[1]), __frcp_rn(e.den[2]));
+        const float3 rA = make_float3(__fdividef(1.0f, e.A[0]), __fdividef(1.0f, e.A[1]), __fdividef(1.0f, e.A[2]));
+        for (uint32_t yb = y0; yb < ye; yb += 32u) {
+            // One row per lane: its covered span.
+            int lo = (int)x0, hi = (int)xe - 1;
+            if (yb + lane < ye) {
+                const float yf = (float)(yb + lane);
+                row_span(e, 0, rA.x, yf, (int)x0, (int)xe - 1, lo, hi);
+                row_span(e, 1, rA.y, yf, (int)x0, (int)xe - 1, lo, hi);
+                row_span(e, 2, rA.z, yf, (int)x0, (int)xe - 1, lo, hi);
+            } else {
+                hi = lo - 1;
+            }
+            const uint32_t cnt = hi >= lo ? (uint32_t)(hi - lo + 1) : 0u;
+            uint32_t incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(FULL, incl, o);
+                if (lane >= (uint32_t)o) incl += v;
+            }
+            const uint32_t total = __shfl_sync(FULL, incl, 31);
+            const uint32_t first = (uint32_t)lo - (incl - cnt);  // column of the row's fragment j: first + j
+            // The covered pixels, 32 at a time: fragment j is in the first row whose inclusive count exceeds it.
+            for (uint32_t b0 = 0; b0 < total; b0 += 32u) {
+                const uint32_t j = b0 + lane;
+                int r = 0, re = 31;
+#pragma unroll
+                for (int it = 0; it < 5; it++) {
+                    const int mid = (r + re) >> 1;
+                    if (__shfl_sync(FULL, incl, mid) > j)
+                        re = mid;
+                    else
+                        r = mid + 1;
+                }
+                const uint32_t x = __shfl_sync(FULL, first, r) + j, y = yb + (uint32_t)r;
+                if (j < total) {
+                    const float xf = (float)x, yf = (float)y;
+                    const float al = div_rcp(edge_eval(e, 0, xf, yf), e.den[0], yr.x);
+                    const float be = div_rcp(edge_eval(e, 1, xf, yf), e.den[1], yr.y);
+                    const float ga = div_rcp(edge_eval(e, 2, xf, yf), e.den[2], yr.z);
+                    const float depth = interp(al, be, ga, dd.x, dd.y, dd.z);
+                    if (depth < clear_depth) atomicMin(vis + (y * width + x), depth_key(depth, seq));
+                }
+            }
+        }
     }
 }
 
