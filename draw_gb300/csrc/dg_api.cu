@@ -747,7 +747,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     job.items = S.d_items;
     job.items_cap = (uint32_t)std::min<size_t>(S.items_cap, 0xFFFFFFF0ull);
     job.queue_cap = (uint32_t)std::min<size_t>(S.queue_cap, (1u << 24) - 1);
-    job.item_units = S.item_units;
+    job.item_log2 = dg_item_log2(S.item_units);
     job.cnt = S.d_counters;
     job.total_px = (uint32_t)total_px;
     job.tile_rows = th;

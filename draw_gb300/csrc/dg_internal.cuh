@@ -55,8 +55,8 @@ __device__ __forceinline__ bool dg_check_range(bool ok, uint32_t* err) {
 // Triangles whose clipped bounding box has at most DgFrameDev.small_max_px
 // pixels go to the small-triangle list, whose entries the queue pass
 // rasterizes one per lane; larger ones go to the raster queue: their bounding
-// box is cut into work items (DgItemGrid) of about 128 * DgJobDev.item_units
-// pixels (default DG_ITEM_UNITS), which the queue pass spreads over all warps. Unless the
+// box is cut into work items (DgItemGrid) of about 2^DgJobDev.item_log2 pixels
+// (128 * item_units, default DG_ITEM_UNITS), which the queue pass spreads over all warps. Unless the
 // tuning fixes it, a frame's threshold is DG_SMALL_MAX_PX, or
 // DG_SMALL_MAX_PX_MICRO when the frame has at least as many triangles as
 // pixels: lanes that each loop over a box of up to 64 pixels pay off only when
@@ -232,26 +232,39 @@ struct alignas(16) DgQueueRec {
 // How the box of a queued triangle is cut into work items: a grid of nx columns
 // of items, each cw x rh pixels (the last ones less). A warp finds the covered
 // span of up to 32 rows at once, so an item is 32 rows high and as wide as
-// keeps it at about 128 * item_units pixels, wider for boxes of fewer rows and
+// keeps it at about its job's item size, wider for boxes of fewer rows and
 // several times 32 rows high for boxes of fewer columns.
 struct DgItemGrid {
     uint32_t cw, rh, nx, n;
 };
-__host__ __device__ inline DgItemGrid dg_item_grid(uint32_t w, uint32_t h, uint32_t item_units) {
-    const uint32_t px = 128u * item_units;
-    uint32_t pw = 1u, ph = 1u;  // box size rounded up to a power of two, at most 32
-    while (pw < w && pw < 32u) pw *= 2u;
-    while (ph < h && ph < 32u) ph *= 2u;
+// lpx: log2 of the pixels per item (7..15, DgJobDev::item_log2). Shifts only:
+// the setup pass evaluates it in its long dependent chain.
+__device__ __forceinline__ DgItemGrid dg_item_grid(uint32_t w, uint32_t h, uint32_t lpx) {
+    auto log2_up = [](uint32_t v) { return 32u - (uint32_t)__clz((int)(v - 1u)); };  // ceil(log2 v), 0 for 1
     DgItemGrid g;
-    g.cw = w <= 32u ? w : px / ph;  // at least 4
-    const uint32_t rows = (px / pw) & ~31u;
-    g.rh = w <= 32u && rows > 32u ? rows : 32u;
-    g.nx = (w + g.cw - 1u) / g.cw;
-    g.n = g.nx * ((h + g.rh - 1u) / g.rh);
+    if (w <= 32u) {
+        const uint32_t lr = max(5u, lpx - log2_up(w));
+        g.cw = w;
+        g.rh = 1u << lr;
+        g.nx = 1u;
+        g.n = (h + g.rh - 1u) >> lr;
+    } else {
+        const uint32_t lc = lpx - (h < 32u ? log2_up(h) : 5u);
+        g.cw = 1u << lc;  // at least 4
+        g.rh = 32u;
+        g.nx = (w + g.cw - 1u) >> lc;
+        g.n = g.nx * ((h + 31u) >> 5);
+    }
     return g;
 }
 
 #define DG_NONE 0xFFFFFFFFu
+// 128 * item_units pixels, rounded down to a power of two.
+inline uint32_t dg_item_log2(uint32_t item_units) {
+    uint32_t l = 7u;
+    while (item_units >>= 1) l++;
+    return l;
+}
 // Job counters (unsigned long long each), each on its own 128-byte line: the
 // hot ones take one atomic per warp or block from every pass, and counters that
 // share a line share one L2 slice, which serializes their updates (measured: the
@@ -300,7 +313,7 @@ struct DgJobDev {
     uint32_t items_cap;
     DgQueueRec* small;      // small-triangle list, rasterized one triangle per lane
     uint32_t small_cap;
-    uint32_t item_units;    // size of the raster work items in 128 pixels (>= 1)
+    uint32_t item_log2;     // log2 of the pixels of a raster work item
     uint32_t total_px;      // pixels of all frames
     uint32_t tile_rows;     // resolve tile height (8, 16 or 32)
     unsigned long long* cnt;  // the job counters (DG_CNT_*, DG_NCOUNTERS words), zero at the start of the job

@@ -400,7 +400,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 const unsigned qmask = __ballot_sync(FULL, nu != 0u);
                 if (qmask) {
                     const uint32_t bw = tr.xhi - tr.xlo + 1u, bh = tr.yhi - tr.ylo + 1u;
-                    const uint32_t ni = nu ? dg_item_grid(bw, bh, job.item_units).n : 0u;
+                    const uint32_t ni = nu ? dg_item_grid(bw, bh, job.item_log2).n : 0u;
                     uint32_t incl = ni, uincl = nu;
     #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
@@ -514,6 +514,11 @@ __global__ void __launch_bounds__(256) k_setup_raster(const DgJobDev job) {
     dev_setup(job);
 }
 
+// Row of pixel k (row-major, k < 4096) of a box whose width's reciprocal is rw:
+// (k + 0.5) / width is at least 0.5 / width from an integer, far more than the
+// error of the product.
+__device__ __forceinline__ uint32_t box_row(uint32_t k, float rw) { return (uint32_t)(((float)k + 0.5f) * rw); }
+
 __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
     __shared__ uint32_t s_sorted[256];             // a group of small triangles in box-size order
     __shared__ uint32_t s_bucket[16];              // their counts, then offsets, per box-size class
@@ -540,8 +545,12 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
     // box-size class (the bit length of the box's pixel count) in shared memory, so
     // that the lanes of a warp loop over boxes of about the same size
     // (block-uniform loop); fewer go in chunks of 32 to single warps, ahead of the
-    // work items.
+    // work items. With fewer than two per warp, a lane's pixel loop would be the
+    // pass's longest chain: they go in pairs, 16 lanes each (a 1283x717 frame of
+    // 679 small triangles: the pass 20.5 -> 12.3 us; 512x512 with 23,500, 1.6 per
+    // warp: 20.5 -> 18.4; ten frames with 50,000, 3.4 per warp: 28.7 -> 32.8).
     const bool sort_small = nsmall >= nwarps * 32u;
+    const bool few_small = nsmall < nwarps * 2u;
     const uint32_t nsgroups = sort_small ? (nsmall + 255u) >> 8 : 0u;
     for (uint32_t gi = blockIdx.x; gi < nsgroups; gi += gridDim.x) {
         if (threadIdx.x < 16u) s_bucket[threadIdx.x] = 0u;
@@ -579,8 +588,25 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
         __syncthreads();  // s_bucket and s_sorted are reused by the next group
     }
     // Work index wi: chunks of 32 small triangles (wi < nchunks), then the work items.
-    const uint32_t nchunks = sort_small ? 0u : (nsmall + 31u) >> 5;
+    const uint32_t nchunks = sort_small ? 0u : few_small ? (nsmall + 1u) >> 1 : (nsmall + 31u) >> 5;
     for (uint32_t wi = warp; wi < nchunks + nitems; wi += nwarps) {
+        if (wi < nchunks && few_small) {
+            const uint32_t i = 2u * wi + (lane >> 4);
+            if (i < nsmall) {
+                const uint4* qs = reinterpret_cast<const uint4*>(job.small + i);
+                const uint4 q0 = __ldcg(qs), q1 = __ldcg(qs + 1);
+                const DgTriRec* R = job.trec + q0.x;
+                EdgeSet e;
+                load_edges(R, e);
+                const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
+                const float rw = __fdividef(1.0f, (float)q1.y);
+                for (uint32_t k = lane & 15u; k < q1.y * q1.z; k += 16u) {
+                    const uint32_t r = box_row(k, rw);
+                    raster_pixel(e, dd.x, dd.y, dd.z, q0.y, q0.w + (k - r * q1.y), q1.x + r, job.frames[q0.z]);
+                }
+            }
+            continue;
+        }
         if (wi < nchunks) {
             const uint32_t i = (wi << 5) + lane;
             if (i < nsmall) {
@@ -610,7 +636,15 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
         const uint32_t width = fr.width;
         const uint32_t xlo = q0.w, ylo = q1.x, w = q1.y, h = q1.z;
         if (!DG_IN_RANGE(w != 0u && xlo + w <= width && ylo + h <= fr.height && q0.x < job.trec_cap, job.err)) continue;
-        const DgItemGrid grid = dg_item_grid(w, h, job.item_units);
+        if (w * h <= 32u) {  // one pixel per lane: cheaper than spans (32 small frames: the pass 77.8 -> 69.6 us)
+            if (lane < w * h) {
+                const uint32_t r = box_row(lane, __fdividef(1.0f, (float)w));
+                raster_pixel(e, dd.x, dd.y, dd.z, seq, xlo + (lane - r * w), ylo + r, fr);
+            }
+            __syncwarp();
+            continue;
+        }
+        const DgItemGrid grid = dg_item_grid(w, h, job.item_log2);
         const uint32_t iy = grid.nx == 1u ? item.y : item.y / grid.nx, ix = item.y - iy * grid.nx;
         const uint32_t x0 = xlo + ix * grid.cw, xe = min(x0 + grid.cw, xlo + w);  // columns [x0, xe)
         const uint32_t y0 = ylo + iy * grid.rh, ye = min(y0 + grid.rh, ylo + h);  // rows [y0, ye)
@@ -1002,7 +1036,11 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     if ((e = dg_launch_transparent(0, job, cfg.tplan, s)) != cudaSuccess) return e;
     if (job.total_tri || job.ntt) {
         NvtxRange r("k_queue_raster");
-        const unsigned qb = cfg.queue_blocks < 1u ? 1u : cfg.queue_blocks;
+        // Blocks beyond a job's possible work only cost their launch: at most a warp per
+        // triangle, and one per 8 pixels for what its triangles' boxes may be cut into
+        // (a 96x64 frame of 200 triangles 24.3 -> 23.0 us).
+        const uint64_t qw = (uint64_t)job.total_tri + job.total_px / 8u + job.total_vtx / 32u;
+        const unsigned qb = grid_for(qw * 32u, cfg.queue_blocks < 1u ? 1u : cfg.queue_blocks);
         if ((e = launch_dependent(k_queue_raster, qb, 256, job, s)) != cudaSuccess) return e;
     }
     if ((e = mark(4)) != cudaSuccess) return e;

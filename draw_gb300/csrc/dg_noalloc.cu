@@ -229,7 +229,7 @@ extern "C" dg_status dg_render_noalloc(const dg_frame_params* p, const dg_device
     job.items = reinterpret_cast<uint2*>(base + kOffQbase);
     job.items_cap = (uint32_t)dg_items_cap(kQueueCap);
     job.queue_cap = kQueueCap;
-    job.item_units = DG_ITEM_UNITS;
+    job.item_log2 = dg_item_log2(DG_ITEM_UNITS);
     job.cnt = reinterpret_cast<unsigned long long*>(base + kOffCounters);
     job.total_px = (uint32_t)npx;
     job.tile_rows = DG_TILE_H;

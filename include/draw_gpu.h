@@ -100,8 +100,8 @@ dg_status dg_ctx_kernel_times(dg_ctx* ctx, float* ms, int32_t n);
 dg_status dg_timeline_read(dg_ctx* ctx, uint64_t* out, int32_t n);
 /* Launch-shape knobs of the raster passes (chosen by dg_autotune below):
  * small_max_px: triangles whose clipped bounding box has at most this many
- * pixels are rasterized one triangle per lane, the others are cut into 32-pixel
- * units spread over all warps (0 = all cut into units, max 4096;
+ * pixels are rasterized one triangle per lane, the others are cut into work
+ * items spread over all warps (0 = all cut into items, max 4096;
  * DG_SMALL_MAX_PX_AUTO, the default: per frame, 64 when the frame has at least
  * as many triangles as pixels, else 16); setup_blocks_per_sm,
  * queue_blocks_per_sm and cull_blocks_per_sm: grid sizes (caps) of those
@@ -109,8 +109,9 @@ dg_status dg_timeline_read(dg_ctx* ctx, uint64_t* out, int32_t n);
  * many triangle records per render (triangles beyond it are shaded from the
  * mesh again in the resolve pass); tile_rows: height of the resolve pass's
  * 32-pixel-wide tiles (8, 16 or 32; 0, the default: per render job, the tallest
- * whose tiles fill 4 resolve blocks per SM, else 8); item_units: 32-pixel units per work item
- * of the queue pass (1..256). Results do not depend on them. */
+ * whose tiles fill 4 resolve blocks per SM, else 8); item_units: box pixels per work item
+ * of the queue pass, in 128 (1..256, rounded down to a power of two). Results do
+ * not depend on them. */
 #define DG_SMALL_MAX_PX_AUTO 0xFFFFFFFFu
 typedef struct {
     uint32_t small_max_px;
@@ -125,7 +126,7 @@ dg_status dg_ctx_set_tuning(dg_ctx* ctx, const dg_tuning* t);
 dg_status dg_ctx_get_tuning(dg_ctx* ctx, dg_tuning* t);
 
 /* Counters of the last render (up to 14): [0] vertices, [1] input triangles, [2] triangles
- * queued for the load-balanced raster pass, [3] their 32-pixel work units, [4] covered
+ * queued for the load-balanced raster pass, [3] their boxes' 32-pixel units, [4] covered
  * pixels (written by resolve), [5] triangles rasterized in place because the queue, the
  * small-triangle list or the triangle records were full, [6] host-to-device bytes of the
  * job descriptor, [7] kernels launched, [8] triangles that passed the cull pass,
