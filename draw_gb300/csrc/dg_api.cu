@@ -374,8 +374,9 @@ dg_status slot_init(dg_ctx* c, JobSlot& s, cudaStream_t stream) {
     s.stream = stream;
     for (int i = 0; i < JobSlot::kStage; i++) DG_CUDA(cudaEventCreateWithFlags(&s.stage_ev[i], cudaEventDisableTiming));
     for (int i = 0; i <= DG_NKERNELS; i++) DG_CUDA(cudaEventCreate(&s.ev[i]));
-    dg_status e = dalloc(&s.d_counters, DG_NCOUNTERS);
+    dg_status e = dalloc(&s.d_counters, 2 * DG_NCOUNTERS);
     if (e) return e;
+    DG_CUDA(cudaMemsetAsync(s.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), stream));
     e = dalloc(&s.d_err, 1);
     if (e) return e;
     DG_CUDA(cudaMemset(s.d_err, 0, 4));
@@ -748,7 +749,8 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     job.items_cap = (uint32_t)std::min<size_t>(S.items_cap, 0xFFFFFFF0ull);
     job.queue_cap = (uint32_t)std::min<size_t>(S.queue_cap, (1u << 24) - 1);
     job.item_log2 = dg_item_log2(S.item_units);
-    job.cnt = S.d_counters;
+    job.cnt = S.d_counters + S.cnt_set * DG_NCOUNTERS;
+    job.cnt_next = S.d_counters + (1 - S.cnt_set) * DG_NCOUNTERS;
     job.total_px = (uint32_t)total_px;
     job.tile_rows = th;
     job.tex = c->d_tex;
@@ -808,8 +810,8 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
 dg_status enqueue_job(JobBuild& B, JobSlot& S, void* d_stage, cudaStream_t stream, bool timing) {
     B.job.frames = (const DgFrameDev*)d_stage;
     B.job.segs = (const DgSegDev*)((uint8_t*)d_stage + B.fbytes);
-    if (!B.job.total_vtx)  // otherwise the first kernel zeroes them
-        DG_CUDA(cudaMemsetAsync(S.d_counters, 0, DG_NCOUNTERS * sizeof(unsigned long long), stream));
+    if (!B.job.total_vtx)  // otherwise the first kernel does
+        DG_CUDA(cudaMemsetAsync(B.job.cnt_next, 0, DG_NCOUNTERS * sizeof(unsigned long long), stream));
     DG_CUDA(dg_launch_job(B.job, B.cfg, stream, timing ? S.ev : nullptr));
     return DG_OK;
 }
@@ -849,6 +851,8 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
         for (size_t i = 0; i < B.segs.size(); i++) inl.segs[i] = B.segs[i];
         inl.nsegs = (uint32_t)B.segs.size();
         B.cfg.inl = &inl;
+        B.cfg.front = B.total_tri > 0 && B.total_tri <= DG_FRONT_MAX_TRI;
+        if (B.cfg.front) B.launches -= 2;
     } else {
         std::memcpy(S.h_stage[k], B.frames.data(), B.fbytes);
         std::memcpy((uint8_t*)S.h_stage[k] + B.fbytes, B.segs.data(), B.sbytes);
@@ -862,7 +866,13 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
     S.last_tile_rows = B.job.tile_rows;
     S.last_small_max_px = B.frames.empty() ? 0 : B.frames[0].small_max_px;
     e = enqueue_job(B, S, S.d_stage[k], S.stream, S.timing);
-    if (e) return e;
+    if (e) {  // part of the job may have run: start over with zero counters
+        cudaMemsetAsync(S.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), S.stream);
+        cudaGetLastError();
+        return e;
+    }
+    S.last_set = S.cnt_set;
+    S.cnt_set ^= 1;
     advance_transparent(c, B);
     if (S.timing) S.ev_valid = true;
     return DG_OK;
@@ -1049,7 +1059,7 @@ dg_status dg_ctx_last_stats(dg_ctx* c, uint64_t* out, int32_t n) {
     JobSlot& S = c->main;
     DG_CUDA(cudaStreamSynchronize(S.stream));
     unsigned long long h[DG_NCOUNTERS];
-    DG_CUDA(cudaMemcpy(h, S.d_counters, sizeof(h), cudaMemcpyDeviceToHost));
+    DG_CUDA(cudaMemcpy(h, S.d_counters + S.last_set * DG_NCOUNTERS, sizeof(h), cudaMemcpyDeviceToHost));
     const uint64_t v[14] = {S.last_vtx,
                             S.last_tri,
                             h[DG_CNT_QUEUE] >> DG_PACK_SHIFT,

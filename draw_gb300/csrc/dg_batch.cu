@@ -130,7 +130,12 @@ dg_status capture(dg_batch* b, const std::vector<Scene*>& sc, const std::vector<
         }
         b->stage_cap = need;
     }
+    // Graph k uses counter set k and zeroes the other one for the next replay.
+    DG_CUDA(cudaMemsetAsync(S.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), S.stream));
+    DG_CUDA(cudaStreamSynchronize(S.stream));
     for (int k = 0; k < 2; k++) {
+        B.job.cnt = S.d_counters + k * DG_NCOUNTERS;
+        B.job.cnt_next = S.d_counters + (1 - k) * DG_NCOUNTERS;
         DG_CUDA(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal));
         cudaError_t ce = cudaMemcpyAsync(b->d_stage[k], b->h_stage[k], need, cudaMemcpyHostToDevice, b->cap);
         dg_status le = ce == cudaSuccess ? enqueue_job(B, S, b->d_stage[k], b->cap, false) : DG_E_CUDA;
@@ -246,7 +251,12 @@ dg_status dg_batch_render(dg_batch* b) {
     DG_CUDA(cudaEventSynchronize(b->done[k]));  // the previous replay of graph k has read its staging
     std::memcpy(b->h_stage[k], B.frames.data(), B.fbytes);
     std::memcpy((uint8_t*)b->h_stage[k] + B.fbytes, B.segs.data(), B.sbytes);
-    DG_CUDA(cudaGraphLaunch(b->exec[k], c->main.stream));
+    const cudaError_t ge = cudaGraphLaunch(b->exec[k], c->main.stream);
+    if (ge != cudaSuccess) {  // the next replay captures again, with zero counters
+        cudaGetLastError();
+        drop_graphs(b);
+        return ge == cudaErrorMemoryAllocation ? DG_E_OOM : DG_E_CUDA;
+    }
     DG_CUDA(cudaEventRecord(b->done[k], c->main.stream));
     advance_transparent(c, B);
     b->replays++;

@@ -648,6 +648,7 @@ __device__ __forceinline__ void wait_previous_kernel() {
 // Hands out n consecutive slots of counter c to every lane of the (converged)
 // warp with one atomic; returns this lane's first slot.
 __device__ __forceinline__ unsigned long long warp_alloc(unsigned long long* c, uint32_t n) {
+    if (__ballot_sync(FULL, n != 0u) == 0u) return 0ull;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t incl = n;
 #pragma unroll
@@ -655,13 +656,9 @@ __device__ __forceinline__ unsigned long long warp_alloc(unsigned long long* c, 
         const uint32_t v = __shfl_up_sync(FULL, incl, o);
         if (lane >= (uint32_t)o) incl += v;
     }
-    const uint32_t total = __shfl_sync(FULL, incl, 31);
     unsigned long long old = 0;
-    if (total != 0u) {
-        if (lane == 31u) old = atomicAdd(c, (unsigned long long)total);
-        old = __shfl_sync(FULL, old, 31);
-    }
-    return old + (incl - n);
+    if (lane == 31u) old = atomicAdd(c, (unsigned long long)incl);
+    return __shfl_sync(FULL, old, 31) + (incl - n);
 }
 
 // Rasterizes a triangle's clipped bounding box on the calling lane alone, row

@@ -176,7 +176,11 @@ struct JobSlot {
     uint32_t tile_rows = 0;  // 0: chosen per job (build_job)
     uint32_t item_units = DG_ITEM_UNITS;
     uint32_t record_limit = 0;
-    unsigned long long* d_counters = nullptr;  // the job counters (DG_CNT_*, DG_NCOUNTERS words)
+    // Two sets of job counters (DG_CNT_*, DG_NCOUNTERS words each): jobs alternate,
+    // and a job's first kernel zeroes the other set for the job after it.
+    unsigned long long* d_counters = nullptr;
+    int cnt_set = 0;   // the next job's set
+    int last_set = 0;  // the last job's set
     uint32_t* d_err = nullptr;
     static const int kStage = 4;  // pinned staging ring for job descriptors
     void* h_stage[kStage] = {};

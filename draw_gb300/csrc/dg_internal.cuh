@@ -283,7 +283,7 @@ inline uint32_t dg_item_log2(uint32_t item_units) {
 #define DG_CNT_TFRAG (10 * DG_CNT_LINE)   // transparent fragments emitted
 #define DG_CNT_TITEMX (11 * DG_CNT_LINE)  // further items of the transparent outputs
 #define DG_CNT_TSLOT (12 * DG_CNT_LINE)   // fragment nodes handed out (chunks of DG_FRAG_CHUNK)
-#define DG_NCOUNTERS (13 * DG_CNT_LINE)   // words of the counter array (k_vertex zeroes them: <= 256)
+#define DG_NCOUNTERS (13 * DG_CNT_LINE)   // words of the counter array
 
 struct DgJobDev {
     const DgFrameDev* frames;
@@ -317,6 +317,7 @@ struct DgJobDev {
     uint32_t total_px;      // pixels of all frames
     uint32_t tile_rows;     // resolve tile height (8, 16 or 32)
     unsigned long long* cnt;  // the job counters (DG_CNT_*, DG_NCOUNTERS words), zero at the start of the job
+    unsigned long long* cnt_next;  // the next job's, which the first kernel zeroes (null: the caller does)
     const DgTexDev* tex;
     uint32_t ntex;          // entries of tex
     uint32_t* err;
@@ -391,6 +392,7 @@ struct DgLaunchCfg {
     unsigned setup_blocks;
     unsigned queue_blocks;
     const DgInlineDesc* inl;  // host memory, read at launch; null: descriptors already on the device
+    bool front;               // with inl: k_front in place of the vertex, cull and setup passes
     DgTransparentPlan tplan;
 };
 // k_vertex's grid cap: its resident blocks (launch bounds 256 x 8), one wave
@@ -398,6 +400,19 @@ struct DgLaunchCfg {
 // headline frame 88.8 -> 87.8 us, the stress frame's vertex pass 64 -> 59 us).
 #define DG_VERTEX_BLOCKS_PER_SM 8u
 #define DG_SETUP_BLOCKS_PER_SM 4u
+// Jobs of one frame whose descriptors travel inline and of at most this many
+// triangles take k_front instead of the vertex, cull and setup passes: it saves
+// two launches and their dependent loads, and computes each vertex once per
+// triangle. Measured, three passes against k_front: 200 triangles 23.6 / 20.1 us
+// a frame, 4,800 38.7 / 33.4, 60,000 34.9 / 31.0, 150,000 38.1 / 37.8, 300,000
+// 53.8 / 55.4, a million 93.8 / 111 us. Blocks of 128 threads: 64 and 256 measured
+// the same or up to 2 us slower.
+#if DG_TIMELINE
+#define DG_FRONT_MAX_TRI 0u  // the timeline shows every pass as a kernel of its own
+#else
+#define DG_FRONT_MAX_TRI 131072u
+#endif
+#define DG_FRONT_THREADS 128u
 #define DG_CLIP_DEFER 512u  // k_setup_raster: clipped survivors a block sets up in its second pass
 // k_queue_raster's grid: 3 waves of its 4 resident blocks per SM. The passes'
 // work items are taken in a fixed strided order, so later waves even out

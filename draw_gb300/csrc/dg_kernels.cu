@@ -77,6 +77,19 @@ __device__ __forceinline__ void timeline_waited(int k) {
 #define DG_TL_WAITED(k) ((void)0)
 #endif
 
+// The plane-sign mask of a vertex: bit p: plane p has f > 0; bit 8 + p: f <= 0.
+__device__ __forceinline__ uint32_t plane_mask(const DgFrameDev& fr, float4 p4) {
+    const V3 p = {p4.x, p4.y, p4.z};
+    uint32_t mask = 0;
+#pragma unroll
+    for (int pl = 0; pl < 6; pl++) {
+        const float f = plane_f(fr, pl, p);
+        if (f > 0.0f) mask |= 1u << pl;
+        if (f <= 0.0f) mask |= 1u << (8 + pl);
+    }
+    return mask;
+}
+
 template <class SEG, class FRM>
 __device__ __forceinline__ void dev_vertex(const DgJobDev& job, uint32_t nsegs, SEG seg, FRM frame) {
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -84,46 +97,42 @@ __device__ __forceinline__ void dev_vertex(const DgJobDev& job, uint32_t nsegs, 
         uint32_t si = last_le(nsegs, v, [&](uint32_t i) { return seg(i).vtx_begin; });
         const DgSegDev& sg = seg(si);
         const DgFrameDev& fr = frame(sg.frame);
-        float4 p4 = __ldg(sg.pos + (v - sg.vtx_begin));
-        V3 p = {p4.x, p4.y, p4.z};
-        uint32_t mask = 0;
-#pragma unroll
-        for (int pl = 0; pl < 6; pl++) {
-            float f = plane_f(fr, pl, p);
-            if (f > 0.0f) mask |= 1u << pl;
-            if (f <= 0.0f) mask |= 1u << (8 + pl);
-        }
+        const float4 p4 = __ldg(sg.pos + (v - sg.vtx_begin));
+        const uint32_t mask = plane_mask(fr, p4);
         job.vrec[v] = vertex_screen(fr, p4, mask);
         job.vmask[v] = (uint16_t)mask;
     }
 }
 
-// Also zeroes the job counters (the later kernels read them only after waiting
-// for this one) and, for a small job, writes the descriptors of its parameter
-// `in` to job.frames and job.segs.
+// A job's first kernel: zeroes the counters of the slot's next job (this job's
+// were zeroed by the job before it) and, for a small job, writes the descriptors
+// of its parameter `in` to job.frames and job.segs.
+__device__ __forceinline__ void begin_job(const DgJobDev& job, const DgInlineDesc& in) {
+    if (blockIdx.x != 0) return;
+    if (job.cnt_next)
+        for (uint32_t i = threadIdx.x; i < DG_NCOUNTERS; i += blockDim.x) job.cnt_next[i] = 0ull;
+    if (in.nsegs) {
+        constexpr uint32_t fw = sizeof(DgFrameDev) / 8, sw = sizeof(DgSegDev) / 8;
+        static_assert(sizeof(DgFrameDev) % 8 == 0 && sizeof(DgSegDev) % 8 == 0, "8-byte words");
+        uint2* fd = reinterpret_cast<uint2*>(const_cast<DgFrameDev*>(job.frames));
+        uint2* sd = reinterpret_cast<uint2*>(const_cast<DgSegDev*>(job.segs));
+        const uint2* fs = reinterpret_cast<const uint2*>(&in.frame);
+        const uint2* ss = reinterpret_cast<const uint2*>(in.segs);
+        for (uint32_t i = threadIdx.x; i < fw + in.nsegs * sw; i += blockDim.x) {
+            if (i < fw)
+                fd[i] = fs[i];
+            else
+                sd[i - fw] = ss[i - fw];
+        }
+    }
+}
+
 __global__ void __launch_bounds__(256, 8) k_vertex(const __grid_constant__ DgJobDev job,
                                                    const __grid_constant__ DgInlineDesc in) {
     DG_TL_BLOCK(0);
     allow_next_kernel();
     DG_TL_WAITED(0);  // the first kernel of a job waits on nothing (a stream-ordered launch)
-    if (blockIdx.x == 0) {
-        static_assert(DG_NCOUNTERS <= 256, "block 0 of k_vertex zeroes the counters");
-        if (threadIdx.x < DG_NCOUNTERS) job.cnt[threadIdx.x] = 0ull;
-        if (in.nsegs) {
-            constexpr uint32_t fw = sizeof(DgFrameDev) / 8, sw = sizeof(DgSegDev) / 8;
-            static_assert(sizeof(DgFrameDev) % 8 == 0 && sizeof(DgSegDev) % 8 == 0, "8-byte words");
-            uint2* fd = reinterpret_cast<uint2*>(const_cast<DgFrameDev*>(job.frames));
-            uint2* sd = reinterpret_cast<uint2*>(const_cast<DgSegDev*>(job.segs));
-            const uint2* fs = reinterpret_cast<const uint2*>(&in.frame);
-            const uint2* ss = reinterpret_cast<const uint2*>(in.segs);
-            for (uint32_t i = threadIdx.x; i < fw + in.nsegs * sw; i += blockDim.x) {
-                if (i < fw)
-                    fd[i] = fs[i];
-                else
-                    sd[i - fw] = ss[i - fw];
-            }
-        }
-    }
+    begin_job(job, in);
     if (in.nsegs)
         dev_vertex(job, in.nsegs, [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; },
                    [&](uint32_t) -> const DgFrameDev& { return in.frame; });
@@ -141,6 +150,16 @@ __global__ void __launch_bounds__(256, 8) k_vertex(const __grid_constant__ DgJob
 // the triangle, so testing them in this order gives the reference's surviving
 // set; the plane tests read only the vertex records' sign masks. Survivors are
 // appended (in any order: the visibility key carries the submission index).
+__device__ __forceinline__ bool outside_planes(uint32_t m) { return ((m >> 8) & 0x3Du) != 0u; }
+// Triangle::calc_normal and get_center; a triangle is skipped when (cam - centre) . n <= 0.
+__device__ __forceinline__ bool faces_camera(const DgFrameDev& fr, V3 a, V3 b, V3 c) {
+    const V3 n = vcross(vsub(b, a), vsub(c, b));
+    const V3 zero = {0.0f, 0.0f, 0.0f};
+    const V3 ctr = vdiv(vadd(vadd(vadd(zero, a), b), c), 3.0f);
+    const V3 cam = {fr.cam[0], fr.cam[1], fr.cam[2]};
+    return !(vdot(vsub(cam, ctr), n) <= 0.0f);
+}
+
 __device__ __forceinline__ void dev_cull(const DgJobDev& job) {
     __shared__ uint32_t s_warp[8];
     __shared__ unsigned long long s_base;
@@ -158,16 +177,10 @@ __device__ __forceinline__ void dev_cull(const DgJobDev& job) {
             const bool ok = DG_IN_RANGE(tp.x < sg.nv && tp.y < sg.nv && tp.z < sg.nv, job.err);
             const uint32_t m = ok ? (uint32_t)__ldg(vm + tp.x) & (uint32_t)__ldg(vm + tp.y) & (uint32_t)__ldg(vm + tp.z)
                                   : 0xFFFFu;
-            if (((m >> 8) & 0x3Du) == 0u) {
+            if (!outside_planes(m)) {
                 const float4 pa = __ldg(sg.pos + tp.x), pb = __ldg(sg.pos + tp.y), pc = __ldg(sg.pos + tp.z);
                 const V3 a = {pa.x, pa.y, pa.z}, b = {pb.x, pb.y, pb.z}, c = {pc.x, pc.y, pc.z};
-                // Triangle::calc_normal and get_center; skip when (cam - centre) . n <= 0
-                const V3 n = vcross(vsub(b, a), vsub(c, b));
-                const V3 zero = {0.0f, 0.0f, 0.0f};
-                const V3 ctr = vdiv(vadd(vadd(vadd(zero, a), b), c), 3.0f);
-                const DgFrameDev& fr = job.frames[sg.frame];
-                const V3 cam = {fr.cam[0], fr.cam[1], fr.cam[2]};
-                keep = !(vdot(vsub(cam, ctr), n) <= 0.0f);
+                keep = faces_camera(job.frames[sg.frame], a, b, c);
             }
         }
         const unsigned kb = __ballot_sync(FULL, keep);
@@ -200,17 +213,24 @@ __global__ void __launch_bounds__(256) k_cull(const DgJobDev job) {
 // clipping, triangle records, bounding boxes and edge functions; tiny
 // triangles are rasterized by their warp, the others are queued
 // (scene/mod.rs:1029-1063, canvas.rs:585-681).
-__device__ __forceinline__ void dev_setup(const DgJobDev& job) {
+// FRONT: the whole front of a small job (k_front): the triangles themselves are
+// looped over, and their vertices' masks and screen positions, the plane and the
+// back-face tests computed here instead of read from k_vertex's and k_cull's
+// results; a triangle's record has its job-wide index.
+template <bool FRONT, class SEG, class FRM>
+__device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, SEG seg, FRM frame) {
     __shared__ uint32_t s_records;  // statistics: record requests of the block
+    __shared__ uint32_t s_surv;     // statistics: survivors of the block's culling (FRONT)
     __shared__ uint32_t s_nclip;    // clipped survivors the block deferred
     __shared__ uint32_t s_clip_i[DG_CLIP_DEFER], s_clip_g[DG_CLIP_DEFER];  // their survivor slots and indices
     if (threadIdx.x == 0) {
         s_records = 0u;
+        s_surv = 0u;
         s_nclip = 0u;
     }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long ns64 = __ldcg(job.cnt + DG_CNT_SURV);
+    const unsigned long long ns64 = FRONT ? job.total_tri : __ldcg(job.cnt + DG_CNT_SURV);
     const uint32_t nsurv = (uint32_t)(ns64 < job.total_tri ? ns64 : job.total_tri);
     // Pass 0 sets up the survivors, strided over the grid, but defers those that
     // need near/far clipping (up to DG_CLIP_DEFER per block) to pass 1, where the
@@ -226,13 +246,13 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
             step = blockDim.x;
         }
         for (uint32_t base = start; base < lim; base += step) {
-            const bool valid = base + lane < lim;
+            bool valid = base + lane < lim;
             uint32_t i = base + lane, g = 0;
             if (pass == 1) {
                 i = valid ? s_clip_i[base + lane] : 0u;
                 g = valid ? s_clip_g[base + lane] : 0u;
             } else if (valid) {
-                g = __ldcg(job.surv + i);
+                g = FRONT ? i : __ldcg(job.surv + i);
             }
             int nout = 0;
             uint32_t si = 0, t = 0, row0 = 0, nrows = 0;
@@ -241,13 +261,38 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
             bool clipped = false;
             ClipProg P;  // built once per clipped triangle, used by every output
             if (valid) {
-                si = seg_of_tri(job, g);
-                const DgSegDev& sg = job.segs[si];
+                si = last_le(nsegs, g, [&](uint32_t k) { return seg(k).tri_begin; });
+                const DgSegDev& sg = seg(si);
                 t = g - sg.tri_begin;
                 tp = __ldg(sg.tri_pos + t);
                 tuv = __ldg(sg.tri_uv + t);  // for the triangle record, loaded alongside the vertex records
                 tnr = __ldg(sg.tri_nrm + t);
-                triangle_vertices(job, sg, job.frames[sg.frame], tp, r);
+                if (FRONT) {
+                    valid = DG_IN_RANGE(tp.x < sg.nv && tp.y < sg.nv && tp.z < sg.nv, job.err);
+                    if (valid) {
+                        const DgFrameDev& fr = frame(sg.frame);
+                        const float4 pa = __ldg(sg.pos + tp.x), pb = __ldg(sg.pos + tp.y), pc = __ldg(sg.pos + tp.z);
+                        const uint32_t ma = plane_mask(fr, pa), mb = plane_mask(fr, pb), mc = plane_mask(fr, pc);
+                        // (in pass 1 these hold again: the triangle passed them in pass 0)
+                        valid = !outside_planes(ma & mb & mc) &&
+                                faces_camera(fr, V3{pa.x, pa.y, pa.z}, V3{pb.x, pb.y, pb.z}, V3{pc.x, pc.y, pc.z});
+                        if (valid) {
+                            r[0] = vertex_screen(fr, pa, ma);
+                            r[1] = vertex_screen(fr, pb, mb);
+                            r[2] = vertex_screen(fr, pc, mc);
+                        }
+                    }
+                } else {
+                    triangle_vertices(job, sg, frame(sg.frame), tp, r);
+                }
+            }
+            if (FRONT && pass == 0) {
+                const unsigned kept = __ballot_sync(FULL, valid);
+                if (kept == 0u) continue;
+                if (lane == 0u) atomicAdd(&s_surv, (uint32_t)__popc(kept));
+            }
+            if (valid) {
+                const DgSegDev& sg = seg(si);
                 const uint32_t m = __float_as_uint(r[0].w) & __float_as_uint(r[1].w) & __float_as_uint(r[2].w);
                 uint32_t dslot = DG_CLIP_DEFER;
                 if ((m & 0x3u) == 0x3u) {
@@ -256,7 +301,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                     s_clip_i[dslot] = i;  // set up in pass 1 (nout stays 0 here)
                     s_clip_g[dslot] = g;
                 } else {
-                    const DgFrameDev& fr = job.frames[sg.frame];
+                    const DgFrameDev& fr = frame(sg.frame);
                     float4 pa = __ldg(sg.pos + tp.x), pb = __ldg(sg.pos + tp.y), pc = __ldg(sg.pos + tp.z);
                     build_clip(fr, V3{pa.x, pa.y, pa.z}, V3{pb.x, pb.y, pb.z}, V3{pc.x, pc.y, pc.z}, P);
                     nout = P.nout;
@@ -265,7 +310,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 }
                 // its vertices need light/halfway vectors for shading (in a DG_FRAME_LAZY
                 // frame an unclipped triangle is marked below, unless its record is lazy)
-                if (nout > 0 && (clipped || !(job.frames[sg.frame].flags & DG_FRAME_LAZY))) {
+                if (nout > 0 && (clipped || !(frame(sg.frame).flags & DG_FRAME_LAZY))) {
                     const uint32_t vv[3] = {sg.vtx_begin + tp.x, sg.vtx_begin + tp.y, sg.vtx_begin + tp.z};
                     for (int k = 0; k < 3; k++) job.vmark[vv[k]] = 1u;  // plain stores: every writer writes 1
                 }
@@ -276,7 +321,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 if (nrows != 0u) {
                     if (r0 + nrows <= job.vrow_extra) {
                         row0 = (uint32_t)r0;
-                        clip_shade_rows(job, job.frames[job.segs[si].frame], P, job.total_vtx + row0);
+                        clip_shade_rows(job, frame(seg(si).frame), P, job.total_vtx + row0);
                     } else {
                         nrows = DG_NONE;  // no room: k_resolve shades these pixels the long way
                     }
@@ -313,8 +358,8 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 tr.xlo = tr.xhi = tr.ylo = tr.yhi = 0;
                 tr.frame = 0;
                 if (has) {
-                    const DgSegDev& sg = job.segs[si];
-                    const DgFrameDev& fr = job.frames[sg.frame];
+                    const DgSegDev& sg = seg(si);
+                    const DgFrameDev& fr = frame(sg.frame);
                     tr.frame = sg.frame;
                     tr.seq = ((sg.seq_base + t) << 2) | (uint32_t)rr;
                     if (!clipped) {
@@ -367,7 +412,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                     uint32_t* cells = nullptr;
                     uint32_t ep = 0, cw = 0, ncx = 0, ncy = 0;
                     if (boxed) {
-                        const DgFrameDev& fm = job.frames[tr.frame];
+                        const DgFrameDev& fm = frame(tr.frame);
                         cells = fm.cells;
                         ep = fm.epoch;
                         cw = fm.tiles_x;
@@ -397,6 +442,12 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 // Queue the large triangles of this output index with one 64-bit atomic per warp: it hands out
                 // the queue records and their work items together; the warp then writes all its
                 // items, each lane taking every 32nd.
+                // The small-triangle list's atomic (one per warp) is issued first, so that its
+                // latency overlaps the queue's.
+                const unsigned smask = __ballot_sync(FULL, small);
+                unsigned long long sold = 0;
+                if (smask && (int)lane == __ffs(smask) - 1)
+                    sold = atomicAdd(job.cnt + DG_CNT_SMALL, (unsigned long long)__popc(smask));
                 const unsigned qmask = __ballot_sync(FULL, nu != 0u);
                 if (qmask) {
                     const uint32_t bw = tr.xhi - tr.xlo + 1u, bh = tr.yhi - tr.ylo + 1u;
@@ -476,15 +527,10 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                             job.items[oib + k] = ofits ? make_uint2(orec, k) : make_uint2(DG_NONE, 0u);
                     }
                 }
-                // Small triangles go to the small-triangle list (one atomic per warp), which the
-                // queue pass rasterizes one triangle per lane.
-                const unsigned smask = __ballot_sync(FULL, small);
+                // Small triangles go to the small-triangle list, which the queue pass rasterizes.
                 if (smask) {
-                    const int leader = __ffs(smask) - 1;
-                    unsigned long long old = 0;
-                    if ((int)lane == leader) old = atomicAdd(job.cnt + DG_CNT_SMALL, (unsigned long long)__popc(smask));
-                    old = __shfl_sync(FULL, old, leader);
-                    const uint64_t slot = old + __popc(smask & ((1u << lane) - 1u));
+                    sold = __shfl_sync(FULL, sold, __ffs(smask) - 1);
+                    const uint64_t slot = sold + __popc(smask & ((1u << lane) - 1u));
                     if (small) {
                         if (slot < job.small_cap) {
                             uint4* qd = reinterpret_cast<uint4*>(job.small + slot);
@@ -498,20 +544,39 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job) {
                 if (inplace) {  // this lane rasterizes the box itself
                     atomicAdd(job.cnt + DG_CNT_INPLACE, 1ull);
                     raster_box(e, tr.da, tr.db, tr.dc, tr.seq, tr.xlo, tr.ylo, tr.xhi - tr.xlo + 1u, tr.yhi - tr.ylo + 1u,
-                               job.frames[tr.frame]);
+                               frame(tr.frame));
                 }
             }
         }
     }
     __syncthreads();
     if (threadIdx.x == 0 && s_records) atomicAdd(job.cnt + DG_CNT_TREC, (unsigned long long)s_records);  // statistics only
+    if (FRONT && threadIdx.x == 0 && s_surv) atomicAdd(job.cnt + DG_CNT_SURV, (unsigned long long)s_surv);
 }
 
-__global__ void __launch_bounds__(256) k_setup_raster(const DgJobDev job) {
+__global__ void __launch_bounds__(256) k_setup_raster(const __grid_constant__ DgJobDev job) {
     DG_TL_BLOCK(2);
     wait_previous_kernel();
     DG_TL_WAITED(2);
-    dev_setup(job);
+    dev_setup<false>(job, job.nsegs, [&](uint32_t i) -> const DgSegDev& { return job.segs[i]; },
+                     [&](uint32_t i) -> const DgFrameDev& { return job.frames[i]; });
+}
+
+// The front of a small job as one kernel instead of three: vertex, cull and setup
+// passes of a few thousand triangles are a few microseconds of launch and
+// dependent loads each. A thread computes its triangle's three vertices itself
+// (about three times the vertex arithmetic of k_vertex); the vertex records that
+// the transparent pass and record-less pixels read are written at the end.
+__global__ void __launch_bounds__(DG_FRONT_THREADS) k_front(const __grid_constant__ DgJobDev job,
+                                                            const __grid_constant__ DgInlineDesc in) {
+    DG_TL_BLOCK(2);
+    allow_next_kernel();
+    DG_TL_WAITED(2);
+    begin_job(job, in);
+    auto seg = [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; };
+    auto frame = [&](uint32_t) -> const DgFrameDev& { return in.frame; };
+    dev_setup<true>(job, in.nsegs, seg, frame);
+    dev_vertex(job, in.nsegs, seg, frame);
 }
 
 // Row of pixel k (row-major, k < 4096) of a box whose width's reciprocal is rw:
@@ -1010,22 +1075,28 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     cudaError_t e;
     auto mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s) : cudaSuccess; };
     if ((e = mark(0)) != cudaSuccess) return e;
-    if (job.total_vtx) {
+    DgInlineDesc none;
+    if (!cfg.inl) none.nsegs = 0;
+    const bool front = cfg.front && cfg.inl && job.total_vtx && job.total_tri;
+    if (job.total_vtx && !front) {
         NvtxRange r("k_vertex");
-        DgInlineDesc none;
-        if (!cfg.inl) none.nsegs = 0;
         const unsigned vb = cfg.vertex_blocks < 1u ? 1u : cfg.vertex_blocks;
         k_vertex<<<grid_for(job.total_vtx, vb), 256, 0, s>>>(job, cfg.inl ? *cfg.inl : none);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if ((e = mark(1)) != cudaSuccess) return e;
-    if (job.total_tri) {
+    if (job.total_tri && !front) {
         NvtxRange r("k_cull");
         const unsigned cb = cfg.cull_blocks < 1u ? 1u : cfg.cull_blocks;
         if ((e = launch_dependent(k_cull, grid_for(job.total_tri, cb), 256, job, s)) != cudaSuccess) return e;
     }
     if ((e = mark(2)) != cudaSuccess) return e;
-    if (job.total_tri) {
+    if (front) {
+        NvtxRange r("k_front");
+        const uint32_t blocks = (job.total_tri + DG_FRONT_THREADS - 1u) / DG_FRONT_THREADS;
+        k_front<<<blocks, DG_FRONT_THREADS, 0, s>>>(job, *cfg.inl);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    } else if (job.total_tri) {
         NvtxRange r("k_setup_raster");
         const unsigned sb = cfg.setup_blocks < 1u ? 1u : cfg.setup_blocks;
         if ((e = launch_dependent(k_setup_raster, grid_for(job.total_tri, sb), 256, job, s)) != cudaSuccess) return e;

@@ -86,7 +86,8 @@ dg_status dg_ctx_set_stream(dg_ctx* ctx, void* stream);
 void* dg_ctx_stream(dg_ctx* ctx);
 /* Per-kernel CUDA-event timing of the last render (ms), up to 5 values: "vertex", "cull",
  * "setup_raster", "queue_raster", "resolve". Enabled with dg_ctx_set_timing(ctx, 1); the
- * events between kernels also stop their launch overlap, so frames are slower meanwhile. */
+ * events between kernels also stop their launch overlap, so frames are slower meanwhile. A
+ * small frame's vertex, cull and setup passes are one kernel, timed as "setup_raster". */
 dg_status dg_ctx_set_timing(dg_ctx* ctx, int32_t enable);
 dg_status dg_ctx_kernel_times(dg_ctx* ctx, float* ms, int32_t n);
 /* Kernel timeline of the render jobs since the last call, in builds made with
