@@ -480,7 +480,7 @@ uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L
     const size_t sv = cap_after(s.surv_cap, s.d_surv, std::max<uint64_t>(T, 1));
     const size_t ro = cap_after(s.rec_of_cap, s.d_rec_of, std::max<uint64_t>(T, 1));
     const size_t tr = cap_after(s.trec_cap, s.d_trec, trec_records(T));
-    return vmask * sizeof(uint16_t) + vrec * sizeof(float4) + vshade * sizeof(float4) + vmark * sizeof(uint8_t) + (q + sm) * sizeof(DgQueueRec) +
+    return vmask * sizeof(uint16_t) + vrec * sizeof(float4) + vshade * sizeof(float4) + vmark * sizeof(uint8_t) + q * sizeof(DgQueueRec) + sm * sizeof(DgSmallRec) +
            qb * sizeof(uint2) + (sv + ro) * sizeof(uint32_t) + tr * sizeof(DgTriRec);
 }
 

@@ -137,7 +137,7 @@ struct JobSlot {
     uint8_t* d_vmark = nullptr;  // zeroed at allocation; the queue pass clears what setup sets
     size_t vmark_cap = 0;
     DgQueueRec* d_queue = nullptr;
-    DgQueueRec* d_small = nullptr;  // small-triangle list
+    DgSmallRec* d_small = nullptr;  // small-triangle list
     size_t small_cap = 0;
     // transparent pass scratch (DgJobDev)
     uint64_t* d_tkey[2] = {};

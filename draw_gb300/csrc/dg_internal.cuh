@@ -53,16 +53,13 @@ __device__ __forceinline__ bool dg_check_range(bool ok, uint32_t* err) {
 #define DG_VIS_EMPTY 0xFFFFFFFFFFFFFFFFull
 
 // Triangles whose clipped bounding box has at most DgFrameDev.small_max_px
-// pixels go to the small-triangle list, whose entries the queue pass
-// rasterizes one per lane; larger ones go to the raster queue: their bounding
-// box is cut into work items (DgItemGrid) of about 2^DgJobDev.item_log2 pixels
-// (128 * item_units, default DG_ITEM_UNITS), which the queue pass spreads over all warps. Unless the
-// tuning fixes it, a frame's threshold is DG_SMALL_MAX_PX, or
-// DG_SMALL_MAX_PX_MICRO when the frame has at least as many triangles as
-// pixels: lanes that each loop over a box of up to 64 pixels pay off only when
-// there are millions of such boxes to sort by size (the 3840x2160 frame of 10M
-// micro triangles 1,533 -> 1,423 us), while a frame of few small triangles
-// waits on its longest lane (the headline frame 88 -> 107 us at 64).
+// pixels go to the small-triangle list, whose entries the queue pass rasterizes
+// 32 at a time per warp, their boxes' pixels numbered together; larger ones go to
+// the raster queue: their bounding box is cut into work items (DgItemGrid) of
+// about 2^DgJobDev.item_log2 pixels (128 * item_units, default DG_ITEM_UNITS),
+// which the queue pass spreads over all warps. Unless the tuning fixes it, a
+// frame's threshold is DG_SMALL_MAX_PX, or DG_SMALL_MAX_PX_MICRO when the frame
+// has at least as many triangles as pixels.
 #define DG_SMALL_MAX_PX 16u
 #define DG_SMALL_MAX_PX_MICRO 64u
 #define DG_UNIT_PX 32u
@@ -218,8 +215,7 @@ struct alignas(16) DgTriRec {
 };
 static_assert(sizeof(DgTriRec) == 192, "triangle record size");
 
-// A triangle queued for the load-balanced raster pass, or an entry of the
-// small-triangle list (32 bytes).
+// A triangle queued for the load-balanced raster pass (32 bytes).
 struct alignas(16) DgQueueRec {
     uint32_t rec;     // its DgTriRec
     uint32_t seq;     // frame-local key low word
@@ -227,6 +223,17 @@ struct alignas(16) DgQueueRec {
     uint32_t xlo, ylo;  // clipped bounding box origin
     uint32_t w, h;      // bounding box size in pixels
     uint32_t pad;
+};
+
+// An entry of the small-triangle list (48 bytes): all that its rasterization
+// reads. Boxes are at most 255 pixels wide and high and end below column and row
+// 65536, frames below 65536 (other triangles are queued).
+struct alignas(16) DgSmallRec {
+    float cx[3], cy[3];  // snapped centres
+    float d[3];          // vertex depths (eye distances)
+    uint32_t seq;        // frame-local key low word
+    uint32_t xy;         // clipped bounding box origin: y << 16 | x
+    uint32_t whf;        // frame << 16 | box height << 8 | box width
 };
 
 // How the box of a queued triangle is cut into work items: a grid of nx columns
@@ -311,7 +318,7 @@ struct DgJobDev {
     DgQueueRec* queue;
     uint2* items;           // work items: (queue record, number in its grid)
     uint32_t items_cap;
-    DgQueueRec* small;      // small-triangle list, rasterized one triangle per lane
+    DgSmallRec* small;      // small-triangle list
     uint32_t small_cap;
     uint32_t item_log2;     // log2 of the pixels of a raster work item
     uint32_t total_px;      // pixels of all frames

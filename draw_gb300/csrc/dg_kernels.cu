@@ -145,10 +145,11 @@ __global__ void __launch_bounds__(256, 8) k_vertex(const __grid_constant__ DgJob
 // Cull pass: one thread per input triangle. A triangle is dropped when one
 // lateral plane has all three vertices at f <= 0 (Triangle::clip_against_planes,
 // scene/mod.rs:59-66), when all three are at f <= 0 for the near plane (the
-// near clip then outputs nothing, :67-87 with ViewPlane::clip :662-690), or when
-// it faces away from the camera (:1016-1027). All three are pure predicates of
-// the triangle, so testing them in this order gives the reference's surviving
-// set; the plane tests read only the vertex records' sign masks. Survivors are
+// near clip then outputs nothing, :67-87 with ViewPlane::clip :662-690), when it
+// faces away from the camera (:1016-1027), or when it is not clipped and provably
+// covers no pixel (covers_nothing). All are pure predicates of the triangle, so
+// testing them in this order leaves every triangle with a fragment; the plane
+// tests read only the vertex records' sign masks. Survivors are
 // appended (in any order: the visibility key carries the submission index).
 __device__ __forceinline__ bool outside_planes(uint32_t m) { return ((m >> 8) & 0x3Du) != 0u; }
 // Triangle::calc_normal and get_center; a triangle is skipped when (cam - centre) . n <= 0.
@@ -180,7 +181,13 @@ __device__ __forceinline__ void dev_cull(const DgJobDev& job) {
             if (!outside_planes(m)) {
                 const float4 pa = __ldg(sg.pos + tp.x), pb = __ldg(sg.pos + tp.y), pc = __ldg(sg.pos + tp.z);
                 const V3 a = {pa.x, pa.y, pa.z}, b = {pb.x, pb.y, pb.z}, c = {pc.x, pc.y, pc.z};
-                keep = faces_camera(job.frames[sg.frame], a, b, c);
+                const DgFrameDev& fr = job.frames[sg.frame];
+                keep = faces_camera(fr, a, b, c);
+                if (keep && (m & 0x3u) == 0x3u) {  // unclipped: the snapped centres are its own
+                    const float4 ra = __ldg(job.vrec + sg.vtx_begin + tp.x), rb = __ldg(job.vrec + sg.vtx_begin + tp.y),
+                                 rc = __ldg(job.vrec + sg.vtx_begin + tp.z);
+                    keep = !covers_nothing(ra.x, ra.y, rb.x, rb.y, rc.x, rc.y, fr.width, fr.height);
+                }
             }
         }
         const unsigned kb = __ballot_sync(FULL, keep);
@@ -213,6 +220,15 @@ __global__ void __launch_bounds__(256) k_cull(const DgJobDev job) {
 // clipping, triangle records, bounding boxes and edge functions; tiny
 // triangles are rasterized by their warp, the others are queued
 // (scene/mod.rs:1029-1063, canvas.rs:585-681).
+__device__ __forceinline__ void store_small(DgSmallRec* s, const RTri& tr) {
+    float4* d = reinterpret_cast<float4*>(s);
+    d[0] = make_float4(tr.ax, tr.bx, tr.cx, tr.ay);
+    d[1] = make_float4(tr.by, tr.cy, tr.da, tr.db);
+    reinterpret_cast<uint4*>(s)[2] =
+        make_uint4(__float_as_uint(tr.dc), tr.seq, (tr.ylo << 16) | tr.xlo,
+                   (tr.frame << 16) | ((tr.yhi - tr.ylo + 1u) << 8) | (tr.xhi - tr.xlo + 1u));
+}
+
 // FRONT: the whole front of a small job (k_front): the triangles themselves are
 // looped over, and their vertices' masks and screen positions, the plane and the
 // back-face tests computed here instead of read from k_vertex's and k_cull's
@@ -280,6 +296,8 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                             r[0] = vertex_screen(fr, pa, ma);
                             r[1] = vertex_screen(fr, pb, mb);
                             r[2] = vertex_screen(fr, pc, mc);
+                            valid = (ma & mb & mc & 0x3u) != 0x3u ||
+                                    !covers_nothing(r[0].x, r[0].y, r[1].x, r[1].y, r[2].x, r[2].y, fr.width, fr.height);
                         }
                     }
                 } else {
@@ -398,7 +416,8 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                         }
                         if (rbase == DG_NONE) {
                             inplace = true;
-                        } else if (px <= fr.small_max_px) {
+                        } else if (px <= fr.small_max_px && tr.xhi < 65536u && tr.yhi < 65536u &&
+                                   tr.xhi - tr.xlo < 255u && tr.yhi - tr.ylo < 255u && tr.frame < 65536u) {
                             small = true;
                         } else {
                             nu = (uint32_t)((px + DG_UNIT_PX - 1u) / DG_UNIT_PX);
@@ -533,9 +552,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                     const uint64_t slot = sold + __popc(smask & ((1u << lane) - 1u));
                     if (small) {
                         if (slot < job.small_cap) {
-                            uint4* qd = reinterpret_cast<uint4*>(job.small + slot);
-                            qd[0] = make_uint4(rbase + (uint32_t)rr, tr.seq, tr.frame, tr.xlo);
-                            qd[1] = make_uint4(tr.ylo, tr.xhi - tr.xlo + 1u, tr.yhi - tr.ylo + 1u, 0u);
+                            store_small(job.small + slot, tr);
                         } else {
                             inplace = true;  // list full
                         }
@@ -579,14 +596,147 @@ __global__ void __launch_bounds__(DG_FRONT_THREADS) k_front(const __grid_constan
     dev_vertex(job, in.nsegs, seg, frame);
 }
 
-// Row of pixel k (row-major, k < 4096) of a box whose width's reciprocal is rw:
+// Row of pixel k (row-major) of a box whose width's reciprocal is rw:
 // (k + 0.5) / width is at least 0.5 / width from an integer, far more than the
-// error of the product.
+// error of the product (boxes of at most 65025 pixels).
 __device__ __forceinline__ uint32_t box_row(uint32_t k, float rw) { return (uint32_t)(((float)k + 0.5f) * rw); }
 
+// An entry of the small-triangle list as the raster reads it.
+struct SmallTri {
+    EdgeSet e;
+    float da, db, dc;
+    uint32_t seq, x0, y0, w, h, frame;
+};
+__device__ __forceinline__ SmallTri load_small(const DgSmallRec* s) {
+    const float4* q = reinterpret_cast<const float4*>(s);
+    const float4 a = __ldcg(q), b = __ldcg(q + 1);
+    const uint4 c = __ldcg(reinterpret_cast<const uint4*>(s) + 2);
+    SmallTri t;
+    make_edges(a.x, a.w, a.y, b.x, a.z, b.y, t.e);
+    t.da = b.z;
+    t.db = b.w;
+    t.dc = __uint_as_float(c.x);
+    t.seq = c.y;
+    t.x0 = c.z & 0xFFFFu;
+    t.y0 = c.z >> 16;
+    t.w = c.w & 0xFFu;
+    t.h = (c.w >> 8) & 0xFFu;
+    t.frame = c.w >> 16;
+    return t;
+}
+
+// A warp's 32 small triangles in shared memory: 24 words each, with a stride of
+// seven 16-byte words so that lanes on different triangles read different banks.
+#define DG_SMALL_STRIDE 7
+#define DG_SMALL_WINDOW 512u  // covered pixels listed at a time
+// Rasterizes entries first .. first + 31 of the small-triangle list. Each lane
+// tests its box's pixels one after another into a mask (edges in registers, one
+// comparison per edge); the covered pixels of all 32 are then listed together
+// and finished one per lane, so that the divisions and the keyed minimum run on
+// full warps (about a fifth of the box pixels are covered, unevenly). Measured
+// for the queue pass on 10M micro triangles and on 32 small frames: 306 and 53
+// us; with the pixels of all boxes numbered together and one per lane, 393 and
+// 57; a lane finishing its own pixels, triangles ordered by box size, 411 and 70
+// (before covers_nothing).
+__device__ __forceinline__ void raster_small_chunk(const DgJobDev& job, uint32_t first, uint32_t nsmall, float4* st,
+                                                   uint16_t* list) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint64_t mask = 0;
+    bool whole = false;  // beyond 64 pixels, or not finite: the whole warp takes it below
+    if (first + lane < nsmall) {
+        const SmallTri t = load_small(job.small + first + lane);
+        const uint32_t n = t.w * t.h;
+        whole = n > 64u || !(t.e.tie & DG_EDGE_FAST);
+        float4* d = st + lane * DG_SMALL_STRIDE;
+        d[0] = make_float4(t.e.A[0], t.e.A[1], t.e.A[2], t.e.B[0]);
+        d[1] = make_float4(t.e.B[1], t.e.B[2], t.e.C[0], t.e.C[1]);
+        d[2] = make_float4(t.e.C[2], t.e.D[0], t.e.D[1], t.e.D[2]);
+        d[3] = make_float4(__uint_as_float((t.y0 << 16) | t.x0), __uint_as_float(t.w), __fdividef(1.0f, (float)t.w),
+                           __uint_as_float(t.frame));
+        d[4] = make_float4(t.e.den[0], t.e.den[1], t.e.den[2], __uint_as_float(t.seq));
+        d[5] = make_float4(t.da, t.db, t.dc, 0.0f);
+        if (!whole) {
+            // covered_signs as one comparison: the edge values are integer-valued (or
+            // infinite), so "> 0, or 0 with the tie bit" is "> 0" or "> -1/2"
+            const float t0 = (t.e.tie & 1u) ? -0.5f : 0.0f, t1 = (t.e.tie & 2u) ? -0.5f : 0.0f,
+                        t2 = (t.e.tie & 4u) ? -0.5f : 0.0f;
+            const float xlo = (float)t.x0, xend = (float)(t.x0 + t.w);
+            float xf = xlo, yf = (float)t.y0;
+            uint32_t m[2] = {0u, 0u};
+#pragma unroll
+            for (int half = 0; half < 2; half++) {
+                const uint32_t end = n < 32u ? n : half == 0 ? 32u : n;
+                for (uint32_t k = 32u * half; k < end; k++) {
+                    const bool in = (edge_eval(t.e, 0, xf, yf) > t0) & (edge_eval(t.e, 1, xf, yf) > t1) &
+                                    (edge_eval(t.e, 2, xf, yf) > t2);
+                    m[half] |= (in ? 1u : 0u) << (k & 31u);
+                    xf += 1.0f;
+                    if (xf == xend) {
+                        xf = xlo;
+                        yf += 1.0f;
+                    }
+                }
+            }
+            mask = ((uint64_t)m[1] << 32) | m[0];
+        }
+    }
+    const uint32_t cnt = (uint32_t)__popcll((long long)mask);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= (uint32_t)o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(FULL, incl, 31);
+    uint32_t pos = incl - cnt;
+    for (uint32_t w0 = 0; w0 < total; w0 += DG_SMALL_WINDOW) {
+        const uint32_t end = min(total, w0 + DG_SMALL_WINDOW);
+        while (mask != 0ull && pos < end) {
+            const uint32_t k = (uint32_t)__ffsll((long long)mask) - 1u;
+            mask &= mask - 1ull;
+            list[pos - w0] = (uint16_t)((lane << 6) | k);
+            pos++;
+        }
+        __syncwarp();
+        for (uint32_t j = w0 + lane; j < end; j += 32u) {
+            const uint32_t at = list[j - w0];
+            const float4* d = st + (at >> 6) * DG_SMALL_STRIDE;
+            const float4 a = d[0], b = d[1], c = d[2], box = d[3], den = d[4], dd = d[5];
+            EdgeSet e;
+            e.A[0] = a.x; e.A[1] = a.y; e.A[2] = a.z; e.B[0] = a.w;
+            e.B[1] = b.x; e.B[2] = b.y; e.C[0] = b.z; e.C[1] = b.w;
+            e.C[2] = c.x; e.D[0] = c.y; e.D[1] = c.z; e.D[2] = c.w;
+            const uint32_t k = at & 63u, xy = __float_as_uint(box.x), dy = box_row(k, box.z);
+            const uint32_t x = (xy & 0xFFFFu) + (k - dy * __float_as_uint(box.y)), y = (xy >> 16) + dy;
+            const float xf = (float)x, yf = (float)y;
+            const DgFrameDev& fr = job.frames[__float_as_uint(box.w)];
+            const float al = fD(edge_eval(e, 0, xf, yf), den.x);
+            const float be = fD(edge_eval(e, 1, xf, yf), den.y);
+            const float ga = fD(edge_eval(e, 2, xf, yf), den.z);
+            const float depth = interp(al, be, ga, dd.x, dd.y, dd.z);
+            if (depth < fr.clear_depth)
+                atomicMin(reinterpret_cast<unsigned long long*>(fr.vis) + (y * fr.width + x),
+                          depth_key(depth, __float_as_uint(den.w)));
+        }
+        __syncwarp();
+    }
+    unsigned big = __ballot_sync(FULL, whole);
+    while (big) {
+        const uint32_t L = (uint32_t)__ffs(big) - 1u;
+        big &= big - 1u;
+        const SmallTri t = load_small(job.small + first + L);
+        const float rw = __fdividef(1.0f, (float)t.w);
+        for (uint32_t k = lane; k < t.w * t.h; k += 32u) {
+            const uint32_t r = box_row(k, rw);
+            raster_pixel(t.e, t.da, t.db, t.dc, t.seq, t.x0 + (k - r * t.w), t.y0 + r, job.frames[t.frame]);
+        }
+        __syncwarp();
+    }
+}
+
 __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
-    __shared__ uint32_t s_sorted[256];             // a group of small triangles in box-size order
-    __shared__ uint32_t s_bucket[16];              // their counts, then offsets, per box-size class
+    __shared__ float4 s_tri[8][32 * DG_SMALL_STRIDE];  // per-warp small triangles
+    __shared__ uint16_t s_list[8][DG_SMALL_WINDOW];    // and their covered pixels
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -605,84 +755,30 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
     const uint32_t nitems = (uint32_t)(ni64 < job.items_cap ? ni64 : job.items_cap);
     const unsigned long long ns64 = __ldcg(job.cnt + DG_CNT_SMALL);
     const uint32_t nsmall = (uint32_t)(ns64 < job.small_cap ? ns64 : job.small_cap);
-    // Small triangles: one per lane, rasterized by that lane. When there are at
-    // least 32 per warp of the grid, a block takes 256 at a time and orders them by
-    // box-size class (the bit length of the box's pixel count) in shared memory, so
-    // that the lanes of a warp loop over boxes of about the same size
-    // (block-uniform loop); fewer go in chunks of 32 to single warps, ahead of the
-    // work items. With fewer than two per warp, a lane's pixel loop would be the
-    // pass's longest chain: they go in pairs, 16 lanes each (a 1283x717 frame of
-    // 679 small triangles: the pass 20.5 -> 12.3 us; 512x512 with 23,500, 1.6 per
-    // warp: 20.5 -> 18.4; ten frames with 50,000, 3.4 per warp: 28.7 -> 32.8).
-    const bool sort_small = nsmall >= nwarps * 32u;
+    // Small triangles go in chunks of 32 to single warps (raster_small_chunk), ahead
+    // of the work items. With fewer than two per warp, a chunk would be the pass's
+    // longest chain: they go in pairs, 16 lanes each (measured with a lane per
+    // triangle: a 1283x717 frame of 679 small triangles, the pass 20.5 -> 12.3 us;
+    // 512x512 with 23,500, 1.6 per warp, 20.5 -> 18.4).
     const bool few_small = nsmall < nwarps * 2u;
-    const uint32_t nsgroups = sort_small ? (nsmall + 255u) >> 8 : 0u;
-    for (uint32_t gi = blockIdx.x; gi < nsgroups; gi += gridDim.x) {
-        if (threadIdx.x < 16u) s_bucket[threadIdx.x] = 0u;
-        __syncthreads();
-        const uint32_t i = (gi << 8) + threadIdx.x;
-        uint32_t cls = 15u, rank = 0;
-        if (i < nsmall) {
-            const uint4 q1 = __ldcg(reinterpret_cast<const uint4*>(job.small + i) + 1);
-            const uint32_t px = q1.y * q1.z;  // at most small_max_px (<= 4096)
-            cls = 32u - __clz(px);            // 0..13
-            rank = atomicAdd(&s_bucket[cls], 1u);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {  // exclusive offsets of the classes; class 15 (no triangle) last
-            uint32_t run = 0;
-            for (uint32_t c = 0; c < 16u; c++) {
-                const uint32_t n = s_bucket[c];
-                s_bucket[c] = run;
-                run += n;
-            }
-        }
-        __syncthreads();
-        if (i < nsmall) s_sorted[s_bucket[cls] + rank] = i;
-        __syncthreads();
-        const uint32_t nin = nsmall - (gi << 8) < 256u ? nsmall - (gi << 8) : 256u;
-        if (threadIdx.x < nin) {
-            const uint4* qs = reinterpret_cast<const uint4*>(job.small + s_sorted[threadIdx.x]);
-            const uint4 q0 = __ldcg(qs), q1 = __ldcg(qs + 1);
-            const DgTriRec* R = job.trec + q0.x;
-            EdgeSet e;
-            load_edges(R, e);
-            const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
-            raster_box(e, dd.x, dd.y, dd.z, q0.y, q0.w, q1.x, q1.y, q1.z, job.frames[q0.z]);
-        }
-        __syncthreads();  // s_bucket and s_sorted are reused by the next group
-    }
-    // Work index wi: chunks of 32 small triangles (wi < nchunks), then the work items.
-    const uint32_t nchunks = sort_small ? 0u : few_small ? (nsmall + 1u) >> 1 : (nsmall + 31u) >> 5;
+    // Work index wi: chunks of small triangles (wi < nchunks), then the work items.
+    const uint32_t nchunks = few_small ? (nsmall + 1u) >> 1 : (nsmall + 31u) >> 5;
     for (uint32_t wi = warp; wi < nchunks + nitems; wi += nwarps) {
         if (wi < nchunks && few_small) {
             const uint32_t i = 2u * wi + (lane >> 4);
             if (i < nsmall) {
-                const uint4* qs = reinterpret_cast<const uint4*>(job.small + i);
-                const uint4 q0 = __ldcg(qs), q1 = __ldcg(qs + 1);
-                const DgTriRec* R = job.trec + q0.x;
-                EdgeSet e;
-                load_edges(R, e);
-                const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
-                const float rw = __fdividef(1.0f, (float)q1.y);
-                for (uint32_t k = lane & 15u; k < q1.y * q1.z; k += 16u) {
+                const SmallTri t = load_small(job.small + i);
+                const float rw = __fdividef(1.0f, (float)t.w);
+                for (uint32_t k = lane & 15u; k < t.w * t.h; k += 16u) {
                     const uint32_t r = box_row(k, rw);
-                    raster_pixel(e, dd.x, dd.y, dd.z, q0.y, q0.w + (k - r * q1.y), q1.x + r, job.frames[q0.z]);
+                    raster_pixel(t.e, t.da, t.db, t.dc, t.seq, t.x0 + (k - r * t.w), t.y0 + r, job.frames[t.frame]);
                 }
             }
+            __syncwarp();
             continue;
         }
         if (wi < nchunks) {
-            const uint32_t i = (wi << 5) + lane;
-            if (i < nsmall) {
-                const uint4* qs = reinterpret_cast<const uint4*>(job.small + i);
-                const uint4 q0 = __ldcg(qs), q1 = __ldcg(qs + 1);
-                const DgTriRec* R = job.trec + q0.x;
-                EdgeSet e;
-                load_edges(R, e);
-                const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
-                raster_box(e, dd.x, dd.y, dd.z, q0.y, q0.w, q1.x, q1.y, q1.z, job.frames[q0.z]);
-            }
+            raster_small_chunk(job, wi << 5, nsmall, s_tri[threadIdx.x >> 5], s_list[threadIdx.x >> 5]);
             continue;
         }
         const uint32_t it = wi - nchunks;

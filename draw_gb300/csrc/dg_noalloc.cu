@@ -43,7 +43,7 @@ constexpr size_t kOffVmark = align_up(kOffVshade + (size_t)(DG_NOALLOC_MAX_VERTI
                                                        DG_NOALLOC_MAX_LIGHTS * 2 * sizeof(float4));
 constexpr size_t kOffQueue = align_up(kOffVmark + (size_t)DG_NOALLOC_MAX_VERTICES * sizeof(uint8_t));
 constexpr size_t kOffSmall = align_up(kOffQueue + (size_t)kQueueCap * sizeof(DgQueueRec));
-constexpr size_t kOffQbase = align_up(kOffSmall + (size_t)kQueueCap * sizeof(DgQueueRec));
+constexpr size_t kOffQbase = align_up(kOffSmall + (size_t)kQueueCap * sizeof(DgSmallRec));
 constexpr size_t kOffSurv = align_up(kOffQbase + (size_t)dg_items_cap(kQueueCap) * sizeof(uint2));
 constexpr size_t kOffRecOf = align_up(kOffSurv + (size_t)DG_NOALLOC_MAX_TRIANGLES * sizeof(uint32_t));
 constexpr size_t kOffTrec = align_up(kOffRecOf + (size_t)DG_NOALLOC_MAX_TRIANGLES * sizeof(uint32_t));
@@ -224,7 +224,7 @@ extern "C" dg_status dg_render_noalloc(const dg_frame_params* p, const dg_device
     job.trec = reinterpret_cast<DgTriRec*>(base + kOffTrec);
     job.trec_cap = kTrecCap;
     job.queue = reinterpret_cast<DgQueueRec*>(base + kOffQueue);
-    job.small = reinterpret_cast<DgQueueRec*>(base + kOffSmall);
+    job.small = reinterpret_cast<DgSmallRec*>(base + kOffSmall);
     job.small_cap = kQueueCap;
     job.items = reinterpret_cast<uint2*>(base + kOffQbase);
     job.items_cap = (uint32_t)dg_items_cap(kQueueCap);
