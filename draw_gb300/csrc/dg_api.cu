@@ -638,7 +638,11 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     }
     e = sync_tex_table(c, S.stream);
     if (e) return e;
-    e = grow(S, &S.d_vmask, &S.vmask_cap, std::max<uint64_t>(total_vtx, 1));
+    // A small job: descriptors as a kernel parameter, and up to DG_FRONT_MAX_TRI
+    // triangles the one-kernel front, which needs no sign masks and no survivor list.
+    B.inline_desc = B.inline_ok && n == 1 && segs.size() <= DG_INLINE_SEGS && total_vtx > 0;
+    B.cfg.front = B.inline_desc && total_tri > 0 && total_tri <= DG_FRONT_MAX_TRI;
+    if (!B.cfg.front) e = grow(S, &S.d_vmask, &S.vmask_cap, std::max<uint64_t>(total_vtx, 1));
     if (e) return e;
     e = grow(S, &S.d_vrec, &S.vrec_cap, std::max<uint64_t>(total_vtx, 1));
     if (e) return e;
@@ -684,7 +688,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         e = grow(S, &S.d_hist, &S.hist_cap, 256 * tiles);
         if (e) return e;
     }
-    e = grow(S, &S.d_surv, &S.surv_cap, std::max<uint64_t>(total_tri, 1));
+    if (!B.cfg.front) e = grow(S, &S.d_surv, &S.surv_cap, std::max<uint64_t>(total_tri, 1));
     if (e) return e;
     e = grow(S, &S.d_rec_of, &S.rec_of_cap, std::max<uint64_t>(total_tri, 1));
     if (e) return e;
@@ -756,7 +760,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     job.tex = c->d_tex;
     job.ntex = (uint32_t)c->tex.size();
     job.err = S.d_err;
-    B.launches = (total_vtx ? 1 : 0) + (total_tri ? 3 : 0) + (total_tiles ? 1 : 0);
+    B.launches = (total_vtx ? 1 : 0) + (total_tri ? 3 : 0) - (B.cfg.front ? 2 : 0) + (total_tiles ? 1 : 0);
     B.cfg.tplan = DgTransparentPlan{};
     if (ntt) {
         job.ntt = (uint32_t)ntt;
@@ -823,6 +827,7 @@ void advance_transparent(dg_ctx* c, const JobBuild& b) {
 dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarget* targets, uint32_t n) {
     if (n == 0) return DG_OK;
     JobBuild B;
+    B.inline_ok = true;
     dg_status e = build_job(c, S, scenes, targets, n, B);
     if (e) return e;
     // job descriptor upload through a pinned staging slot
@@ -830,29 +835,30 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
     const int k = S.stage;
     S.stage = (S.stage + 1) % JobSlot::kStage;
     DG_CUDA(cudaEventSynchronize(S.stage_ev[k]));
+    const size_t stage_cap = std::max<size_t>(need * 2, 64 * 1024);
     if (S.stage_cap[k] < need) {
-        if (S.h_stage[k]) cudaFreeHost(S.h_stage[k]);
         dfree(S.d_stage[k]);
-        S.h_stage[k] = nullptr;
         S.stage_cap[k] = 0;
-        size_t cap = std::max<size_t>(need * 2, 64 * 1024);
-        DG_CUDA(cudaMallocHost(&S.h_stage[k], cap));
-        e = dalloc((uint8_t**)&S.d_stage[k], cap);
+        e = dalloc((uint8_t**)&S.d_stage[k], stage_cap);
         if (e) return e;
-        S.stage_cap[k] = cap;
+        S.stage_cap[k] = stage_cap;
+    }
+    if (!B.inline_desc && S.h_stage_cap[k] < need) {
+        if (S.h_stage[k]) cudaFreeHost(S.h_stage[k]);
+        S.h_stage[k] = nullptr;
+        S.h_stage_cap[k] = 0;
+        DG_CUDA(cudaMallocHost(&S.h_stage[k], stage_cap));
+        S.h_stage_cap[k] = stage_cap;
     }
     // A small job's descriptors go to the device as a kernel parameter (k_vertex
     // writes them to the staging buffer); larger ones are copied.
     DgInlineDesc inl;
-    const bool inline_desc = B.frames.size() == 1 && B.segs.size() <= DG_INLINE_SEGS && B.total_vtx > 0;
-    if (inline_desc) {
+    if (B.inline_desc) {
         std::memset(&inl, 0, sizeof(inl));
         inl.frame = B.frames[0];
         for (size_t i = 0; i < B.segs.size(); i++) inl.segs[i] = B.segs[i];
         inl.nsegs = (uint32_t)B.segs.size();
         B.cfg.inl = &inl;
-        B.cfg.front = B.total_tri > 0 && B.total_tri <= DG_FRONT_MAX_TRI;
-        if (B.cfg.front) B.launches -= 2;
     } else {
         std::memcpy(S.h_stage[k], B.frames.data(), B.fbytes);
         std::memcpy((uint8_t*)S.h_stage[k] + B.fbytes, B.segs.data(), B.sbytes);

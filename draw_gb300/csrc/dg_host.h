@@ -185,7 +185,8 @@ struct JobSlot {
     static const int kStage = 4;  // pinned staging ring for job descriptors
     void* h_stage[kStage] = {};
     void* d_stage[kStage] = {};
-    size_t stage_cap[kStage] = {};
+    size_t stage_cap[kStage] = {};    // bytes of d_stage
+    size_t h_stage_cap[kStage] = {};  // bytes of h_stage (inline descriptors need none)
     cudaEvent_t stage_ev[kStage] = {};
     int stage = 0;
     bool timing = false;
@@ -257,12 +258,14 @@ dg_status launch_frames(dg_ctx* c, JobSlot& s, Scene* const* scenes, const Frame
 // bytes uploaded before the kernels run), the job descriptor the kernels take
 // by value (its frames/segs pointers are set by enqueue_job) and the grid sizes.
 struct JobBuild {
+    bool inline_ok = false;  // set by a caller that can pass the descriptors of a small job inline
     std::vector<DgFrameDev> frames;
     std::vector<DgSegDev> segs;
     size_t fbytes = 0, sbytes = 0;
     DgJobDev job{};
     DgLaunchCfg cfg{};
     uint64_t total_vtx = 0, total_tri = 0, launches = 0;
+    bool inline_desc = false;  // the descriptors go as k_vertex's (k_front's) parameter
     std::vector<int32_t> transparent_objects;  // objects whose transparent order the job advances
 };
 // Host frame setup of every frame (camera basis, matrix, view planes) and the

@@ -90,7 +90,7 @@ __device__ __forceinline__ uint32_t plane_mask(const DgFrameDev& fr, float4 p4) 
     return mask;
 }
 
-template <class SEG, class FRM>
+template <bool MASKS, class SEG, class FRM>
 __device__ __forceinline__ void dev_vertex(const DgJobDev& job, uint32_t nsegs, SEG seg, FRM frame) {
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < job.total_vtx; v += stride) {
@@ -100,7 +100,7 @@ __device__ __forceinline__ void dev_vertex(const DgJobDev& job, uint32_t nsegs, 
         const float4 p4 = __ldg(sg.pos + (v - sg.vtx_begin));
         const uint32_t mask = plane_mask(fr, p4);
         job.vrec[v] = vertex_screen(fr, p4, mask);
-        job.vmask[v] = (uint16_t)mask;
+        if (MASKS) job.vmask[v] = (uint16_t)mask;
     }
 }
 
@@ -134,10 +134,10 @@ __global__ void __launch_bounds__(256, 8) k_vertex(const __grid_constant__ DgJob
     DG_TL_WAITED(0);  // the first kernel of a job waits on nothing (a stream-ordered launch)
     begin_job(job, in);
     if (in.nsegs)
-        dev_vertex(job, in.nsegs, [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; },
+        dev_vertex<true>(job, in.nsegs, [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; },
                    [&](uint32_t) -> const DgFrameDev& { return in.frame; });
     else
-        dev_vertex(job, job.nsegs, [&](uint32_t i) -> const DgSegDev& { return job.segs[i]; },
+        dev_vertex<true>(job, job.nsegs, [&](uint32_t i) -> const DgSegDev& { return job.segs[i]; },
                    [&](uint32_t i) -> const DgFrameDev& { return job.frames[i]; });
 }
 
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(DG_FRONT_THREADS) k_front(const __grid_constan
     auto seg = [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; };
     auto frame = [&](uint32_t) -> const DgFrameDev& { return in.frame; };
     dev_setup<true>(job, in.nsegs, seg, frame);
-    dev_vertex(job, in.nsegs, seg, frame);
+    dev_vertex<false>(job, in.nsegs, seg, frame);
 }
 
 // Row of pixel k (row-major) of a box whose width's reciprocal is rw:
