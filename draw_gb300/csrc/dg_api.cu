@@ -506,8 +506,8 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     // Measured: 256x256 frames 57 -> 41 us (8 rows), 512x512 71 -> 51 us (8 rows),
     // 800x600 47 -> 40 us (16 rows), 1920x1080 best at 32 rows.
     uint32_t th = S.tile_rows;
+    const uint64_t slots = (uint64_t)DG_RESOLVE_BLOCKS_PER_SM * (uint64_t)(c->nsm > 0 ? c->nsm : 1);
     if (th == 0) {
-        const uint64_t slots = 4ull * (uint64_t)(c->nsm > 0 ? c->nsm : 1);
         th = 8;
         for (uint32_t cand : {32u, 16u}) {
             uint64_t tiles = 0;
@@ -757,6 +757,10 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     job.cnt_next = S.d_counters + (1 - S.cnt_set) * DG_NCOUNTERS;
     job.total_px = (uint32_t)total_px;
     job.tile_rows = th;
+    // Up to twice as many 32-row tiles as resident blocks: how many of them are reached
+    // decides between whole tiles and strips (k_resolve_split). Strips of 8 rows pay
+    // when they too fit about two waves, so below half the resident blocks.
+    job.split_below = S.tile_rows == 0 && th == 32 && total_tiles < 2 * slots ? (uint32_t)(slots / 2) : 0u;
     job.tex = c->d_tex;
     job.ntex = (uint32_t)c->tex.size();
     job.err = S.d_err;

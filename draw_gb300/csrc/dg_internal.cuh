@@ -290,7 +290,8 @@ inline uint32_t dg_item_log2(uint32_t item_units) {
 #define DG_CNT_TFRAG (10 * DG_CNT_LINE)   // transparent fragments emitted
 #define DG_CNT_TITEMX (11 * DG_CNT_LINE)  // further items of the transparent outputs
 #define DG_CNT_TSLOT (12 * DG_CNT_LINE)   // fragment nodes handed out (chunks of DG_FRAG_CHUNK)
-#define DG_NCOUNTERS (13 * DG_CNT_LINE)   // words of the counter array
+#define DG_CNT_CELLS (13 * DG_CNT_LINE)   // reached cells (jobs with split_below)
+#define DG_NCOUNTERS (14 * DG_CNT_LINE)   // words of the counter array
 
 struct DgJobDev {
     const DgFrameDev* frames;
@@ -323,6 +324,7 @@ struct DgJobDev {
     uint32_t item_log2;     // log2 of the pixels of a raster work item
     uint32_t total_px;      // pixels of all frames
     uint32_t tile_rows;     // resolve tile height (8, 16 or 32)
+    uint32_t split_below;   // not 0: k_resolve_split takes strips below this many reached cells (tile_rows is 32)
     unsigned long long* cnt;  // the job counters (DG_CNT_*, DG_NCOUNTERS words), zero at the start of the job
     unsigned long long* cnt_next;  // the next job's, which the first kernel zeroes (null: the caller does)
     const DgTexDev* tex;
@@ -427,6 +429,7 @@ struct DgLaunchCfg {
 // 100k-triangle sphere 50.4 -> 46.4 us, the headline frame 89.4 -> 89.1 us).
 #define DG_QUEUE_BLOCKS_PER_SM 12u
 #define DG_CULL_BLOCKS_PER_SM 32u
+#define DG_RESOLVE_BLOCKS_PER_SM 4u  // resident blocks of the resolve pass
 #define DG_NKERNELS 5  // vertex, cull, setup_raster, queue_raster, resolve (+ the transparent pass)
 #define DG_SORT_TILE 4096u  // keys per radix-sort tile (256 threads x 16)
 // Launches the whole pipeline of one job on stream s. ev, if not null, holds

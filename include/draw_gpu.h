@@ -110,7 +110,8 @@ dg_status dg_timeline_read(dg_ctx* ctx, uint64_t* out, int32_t n);
  * many triangle records per render (triangles beyond it are shaded from the
  * mesh again in the resolve pass); tile_rows: height of the resolve pass's
  * 32-pixel-wide tiles (8, 16 or 32; 0, the default: per render job, the tallest
- * whose tiles fill 4 resolve blocks per SM, else 8); item_units: box pixels per work item
+ * whose tiles fill 4 resolve blocks per SM, else 8; a job of 32-row tiles that its triangles
+ * reach few of takes them in strips); item_units: box pixels per work item
  * of the queue pass, in 128 (1..256, rounded down to a power of two). Results do
  * not depend on them. */
 #define DG_SMALL_MAX_PX_AUTO 0xFFFFFFFFu
