@@ -400,6 +400,8 @@ void slot_free(JobSlot& s) {
     s.tsort_cap = s.tout_cap = s.titem_cap = s.fnode_cap = s.fhead_cap = s.hist_cap = 0;
     dfree(s.d_items);
     dfree(s.d_surv);
+    dfree(s.d_rest);
+    s.rest_cap = 0;
     dfree(s.d_rec_of);
     dfree(s.d_trec);
     dfree(s.d_trec_w);
@@ -553,11 +555,12 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         any_persp = any_persp || f.flags != 0u;
         {
             // At least as many opaque triangles as pixels, and a light/halfway table
-            // (32 bytes per vertex and light) beyond the L2: the small triangles'
-            // vertices get no rows, and their shading computes the vectors for the
-            // pixels they win. Measured: the 3840x2160 frame of 10M micro triangles and
-            // 4 lights gains 5% (most of its triangles win no pixel); a 256x256 frame of
-            // a 300k-triangle mesh and 1 light (a 5 MB table) lost 14%, so it keeps rows.
+            // (32 bytes per vertex and light) beyond the L2: the small triangles get no
+            // rows and no records, and the pixels they win are shaded from the mesh.
+            // Measured without the rows alone: the 3840x2160 frame of 10M micro
+            // triangles and 4 lights gained 5% (most of its triangles win no pixel); a
+            // 256x256 frame of a 300k-triangle mesh and 1 light (a 5 MB table) lost 14%,
+            // so it keeps both. k_setup_lean has the figures without the records.
             uint64_t frame_tris = 0, frame_vtx = 0;
             for (int32_t oid : s.objects) {
                 frame_tris += c->objects[oid].ntri_opaque;
@@ -642,6 +645,14 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     // triangles the one-kernel front, which needs no sign masks and no survivor list.
     B.inline_desc = B.inline_ok && n == 1 && segs.size() <= DG_INLINE_SEGS && total_vtx > 0;
     B.cfg.front = B.inline_desc && total_tri > 0 && total_tri <= DG_FRONT_MAX_TRI;
+    if (B.cfg.front && any_lazy) {  // the one-kernel front writes full records
+        any_lazy = false;
+        frames[0].flags &= ~DG_FRAME_LAZY;
+    }
+    if (any_lazy) {
+        e = grow(S, &S.d_rest, &S.rest_cap, total_tri);
+        if (e) return e;
+    }
     if (!B.cfg.front) e = grow(S, &S.d_vmask, &S.vmask_cap, std::max<uint64_t>(total_vtx, 1));
     if (e) return e;
     e = grow(S, &S.d_vrec, &S.vrec_cap, std::max<uint64_t>(total_vtx, 1));
@@ -741,10 +752,12 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     job.trec_w = any_persp ? S.d_trec_w : nullptr;
     job.ext = any_persp ? 1u : 0u;
     job.lazy = any_lazy ? 1u : 0u;
+    job.rest = any_lazy ? S.d_rest : nullptr;
     for (const TexMap& t : c->tex)
         if (t.filter != DG_FILTER_NEAREST) job.ext = 1u;
     job.ttrec_w = any_persp && ntt ? S.d_ttrec_w : nullptr;
     job.trec_cap = (uint32_t)std::min<size_t>(S.trec_cap, 0xFFFFFFF0ull);
+    if (any_lazy) job.trec_cap = std::min(job.trec_cap, DG_LEAN - 1u);
     if (S.record_limit) job.trec_cap = std::min(job.trec_cap, S.record_limit);
     job.queue = S.d_queue;
     job.small = S.d_small;
@@ -764,7 +777,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     job.tex = c->d_tex;
     job.ntex = (uint32_t)c->tex.size();
     job.err = S.d_err;
-    B.launches = (total_vtx ? 1 : 0) + (total_tri ? 3 : 0) - (B.cfg.front ? 2 : 0) + (total_tiles ? 1 : 0);
+    B.launches = (total_vtx ? 1 : 0) + (total_tri ? 3 : 0) + (any_lazy ? 1 : 0) - (B.cfg.front ? 2 : 0) + (total_tiles ? 1 : 0);
     B.cfg.tplan = DgTransparentPlan{};
     if (ntt) {
         job.ntt = (uint32_t)ntt;
@@ -809,6 +822,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     B.cfg.vertex_blocks = (unsigned)c->nsm * DG_VERTEX_BLOCKS_PER_SM;
     B.cfg.cull_blocks = (unsigned)c->nsm * S.cull_blocks_per_sm;
     B.cfg.setup_blocks = (unsigned)c->nsm * S.setup_blocks_per_sm;
+    B.cfg.lean_blocks = (unsigned)c->nsm * DG_LEAN_BLOCKS_PER_SM;
     B.cfg.queue_blocks = (unsigned)c->nsm * S.queue_blocks_per_sm;
     B.total_vtx = total_vtx;
     B.total_tri = total_tri;

@@ -921,40 +921,71 @@ __device__ __forceinline__ const float4* shade_row(const DgJobDev& job, uint32_t
     return job.vshade + (uint64_t)row * (job.shade_stride * 2u) + l * 2u;
 }
 
-// Shades the winning fragment of pixel (x, y) from its triangle record:
-// canvas.rs:682-741.
-// World position of job vertex v (the segment that holds it, then its position).
-__device__ __forceinline__ V3 job_vertex(const DgJobDev& job, uint32_t v) {
-    const uint32_t si = last_le(job.nsegs, v, [&](uint32_t i) { return job.segs[i].vtx_begin; });
-    const DgSegDev& sg = job.segs[si];
-    const float4 p4 = __ldg(sg.pos + (v - sg.vtx_begin));
-    return V3{p4.x, p4.y, p4.z};
+// The segment of frame fr that holds submission index tl (triangles of the frame).
+__device__ __forceinline__ const DgSegDev& seg_of_seq(const DgJobDev& job, const DgFrameDev& fr, uint32_t tl) {
+    return job.segs[fr.seg_begin +
+                    last_le(fr.seg_count, tl, [&](uint32_t i) { return job.segs[fr.seg_begin + i].seq_base; })];
 }
 
+// Shades the winning fragment of pixel (x, y) from its triangle record:
+// canvas.rs:682-741.
 // Wp (frames with DG_FRAME_PERSPECTIVE, else null): the record's inv_w3. EXT
 // as for shade_colour (false: the reference's interpolation and fetch only).
-// LAZY: the record may carry DG_TRI_LAZY, and then the light/halfway vectors of
-// its three vertices are computed here from their positions (shade_vertex's
-// operations) instead of read from job.vshade.
+// LAZY: `lean`, if not null, is the small-list entry of a triangle without a
+// record (R is not read): its edges are set up here again, its attributes and
+// material gathered from the mesh, and the light/halfway vectors of its vertices
+// computed from their positions, all by the operations that fill records and
+// rows, so the values are identical.
 template <bool EXT, bool LAZY>
 __device__ __forceinline__ uint32_t shade_from_record(const DgJobDev& job, const DgFrameDev& fr, const DgTriRec* R,
                                                       uint32_t x, uint32_t y, const float* inv255,
                                                       const DgTexDev* stex, float& depth_out, int& errc,
-                                                      const float4* Wp) {
+                                                      const float4* Wp, const DgSmallRec* lean) {
     errc = DG_OK;
+    const bool from_mesh = LAZY && lean != nullptr;
     EdgeSet e;
-    load_edges(R, e);
-    const float4* q = reinterpret_cast<const float4*>(R);
-    const float4 dd = __ldg(q + 4), fu = __ldg(q + 5), fv = __ldg(q + 6);
-    const float4 fx = __ldg(q + 7), fy = __ldg(q + 8), fz = __ldg(q + 9);
-    const uint4 rows = __ldg(reinterpret_cast<const uint4*>(R) + 10);
-    const uint4 last = __ldg(reinterpret_cast<const uint4*>(R) + 11);
+    float4 dd, fu, fv, fx, fy, fz;
+    uint4 rows, last;
+    V3 va = {0.0f, 0.0f, 0.0f}, vb = va, vc = va;  // vertex positions (from_mesh)
+    if (!from_mesh) {
+        load_edges(R, e);
+        const float4* q = reinterpret_cast<const float4*>(R);
+        dd = __ldg(q + 4), fu = __ldg(q + 5), fv = __ldg(q + 6);
+        fx = __ldg(q + 7), fy = __ldg(q + 8), fz = __ldg(q + 9);
+        rows = __ldg(reinterpret_cast<const uint4*>(R) + 10);
+        last = __ldg(reinterpret_cast<const uint4*>(R) + 11);
+    } else {
+        const float4* q = reinterpret_cast<const float4*>(lean);
+        const float4 s0 = __ldg(q), s1 = __ldg(q + 1);
+        const uint4 s2 = __ldg(reinterpret_cast<const uint4*>(lean) + 2);
+        const uint32_t tl = s2.y >> 2;
+        const DgSegDev& sg = seg_of_seq(job, fr, tl);
+        const uint32_t t = tl - sg.seq_base;
+        const uint4 tp = __ldg(sg.tri_pos + t), tuv = __ldg(sg.tri_uv + t), tnr = __ldg(sg.tri_nrm + t);
+        make_edges(s0.x, s0.w, s0.y, s1.x, s0.z, s1.y, e);
+        const float2 u0 = __ldg(sg.uv + tuv.x), u1 = __ldg(sg.uv + tuv.y), u2 = __ldg(sg.uv + tuv.z);
+        const float4 n0 = __ldg(sg.nrm + tnr.x), n1 = __ldg(sg.nrm + tnr.y), n2 = __ldg(sg.nrm + tnr.z);
+        const float4 pa = __ldg(sg.pos + tp.x), pb = __ldg(sg.pos + tp.y), pc = __ldg(sg.pos + tp.z);
+        float mw[9];
+        mat_words(sg, tp.w, mw, last, job);
+        dd = make_float4(s1.z, s1.w, __uint_as_float(s2.x), mw[0]);
+        fu = make_float4(u0.x, u1.x, u2.x, mw[1]);
+        fv = make_float4(u0.y, u1.y, u2.y, mw[2]);
+        fx = make_float4(n0.x, n1.x, n2.x, mw[3]);
+        fy = make_float4(n0.y, n1.y, n2.y, mw[4]);
+        fz = make_float4(n0.z, n1.z, n2.z, mw[5]);
+        rows = make_uint4(0u, 0u, 0u, __float_as_uint(mw[6]));
+        va = V3{pa.x, pa.y, pa.z};
+        vb = V3{pb.x, pb.y, pb.z};
+        vc = V3{pc.x, pc.y, pc.z};
+    }
     const float xf = (float)x, yf = (float)y;
     float al = fD(edge_eval(e, 0, xf, yf), e.den[0]);
     float be = fD(edge_eval(e, 1, xf, yf), e.den[1]);
     float ga = fD(edge_eval(e, 2, xf, yf), e.den[2]);
     depth_out = interp(al, be, ga, dd.x, dd.y, dd.z);
-    if (EXT && Wp) persp_weights(al, be, ga, __ldg(Wp));  // coverage and depth keep the screen-space weights
+    if (EXT && (Wp || (from_mesh && (fr.flags & DG_FRAME_PERSPECTIVE))))  // coverage and depth keep the screen-space weights
+        persp_weights(al, be, ga, from_mesh ? inv_w3(fr, va, vb, vc) : __ldg(Wp));
     const float pu = interp(al, be, ga, fu.x, fu.y, fu.z);
     const float pv = interp(al, be, ga, fv.x, fv.y, fv.z);
     const V3 pn = {interp(al, be, ga, fx.x, fx.y, fx.z), interp(al, be, ga, fy.x, fy.y, fy.z),
@@ -965,37 +996,37 @@ __device__ __forceinline__ uint32_t shade_from_record(const DgJobDev& job, const
     m.ks = V3{__uint_as_float(rows.w), __uint_as_float(last.x), __uint_as_float(last.y)};
     m.map_ka = last.z;
     m.map_kd = last.w;
-    const bool lazy = LAZY && (e.tie & DG_TRI_LAZY) != 0u;
+    V3 ea = va, eb = vb, ec = vc;  // the vertices' eye vectors
+    if (from_mesh) {
+        const V3 cam = {fr.cam[0], fr.cam[1], fr.cam[2]};
+        ea = vnormalized(vsub(va, cam));
+        eb = vnormalized(vsub(vb, cam));
+        ec = vnormalized(vsub(vc, cam));
+    }
     auto lv = [&](uint32_t l, V3& lt, V3& h) {
-        float4 a, b, c, a1, b1, c1;
-        if (LAZY && lazy) {
-            // each vertex again per light (positions are cached loads): nothing is
-            // held across the lights, which keeps the registers of the common path
-            const V3 cam = {fr.cam[0], fr.cam[1], fr.cam[2]};
-            auto vtx = [&](uint32_t v, float4& o0, float4& o1) {
-                const V3 p = job_vertex(job, v);
-                V3 t, hh;
-                light_halfway(fr, p, vnormalized(vsub(p, cam)), l, t, hh);
-                o0 = make_float4(t.x, t.y, t.z, hh.x);
-                o1 = make_float4(hh.y, hh.z, 0.0f, 0.0f);
-            };
-            vtx(rows.x, a, a1);
-            vtx(rows.y, b, b1);
-            vtx(rows.z, c, c1);
-        } else {
-            if (DG_CHECKED) {
-                const uint32_t nrow = job.total_vtx + job.vrow_extra + 6u * job.ntt;
-                if (!DG_IN_RANGE(rows.x < nrow && rows.y < nrow && rows.z < nrow, job.err)) {
-                    lt = h = V3{0.0f, 0.0f, 0.0f};
-                    return;
-                }
-            }
-            const float4* pa = shade_row(job, rows.x, l);
-            const float4* pb = shade_row(job, rows.y, l);
-            const float4* pc = shade_row(job, rows.z, l);
-            a = __ldg(pa), b = __ldg(pb), c = __ldg(pc);
-            a1 = __ldg(pa + 1), b1 = __ldg(pb + 1), c1 = __ldg(pc + 1);
+        if (from_mesh) {
+            V3 la, ha, lb, hb, lc, hc;
+            light_halfway(fr, va, ea, l, la, ha);
+            light_halfway(fr, vb, eb, l, lb, hb);
+            light_halfway(fr, vc, ec, l, lc, hc);
+            lt = V3{interp(al, be, ga, la.x, lb.x, lc.x), interp(al, be, ga, la.y, lb.y, lc.y),
+                    interp(al, be, ga, la.z, lb.z, lc.z)};
+            h = V3{interp(al, be, ga, ha.x, hb.x, hc.x), interp(al, be, ga, ha.y, hb.y, hc.y),
+                   interp(al, be, ga, ha.z, hb.z, hc.z)};
+            return;
         }
+        if (DG_CHECKED) {
+            const uint32_t nrow = job.total_vtx + job.vrow_extra + 6u * job.ntt;
+            if (!DG_IN_RANGE(rows.x < nrow && rows.y < nrow && rows.z < nrow, job.err)) {
+                lt = h = V3{0.0f, 0.0f, 0.0f};
+                return;
+            }
+        }
+        const float4* pa = shade_row(job, rows.x, l);
+        const float4* pb = shade_row(job, rows.y, l);
+        const float4* pc = shade_row(job, rows.z, l);
+        const float4 a = __ldg(pa), b = __ldg(pb), c = __ldg(pc);
+        const float4 a1 = __ldg(pa + 1), b1 = __ldg(pb + 1), c1 = __ldg(pc + 1);
         lt = V3{interp(al, be, ga, a.x, b.x, c.x), interp(al, be, ga, a.y, b.y, c.y),
                 interp(al, be, ga, a.z, b.z, c.z)};
         h = V3{interp(al, be, ga, a.w, b.w, c.w), interp(al, be, ga, a1.x, b1.x, c1.x),

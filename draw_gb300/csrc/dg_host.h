@@ -161,6 +161,8 @@ struct JobSlot {
     size_t items_cap = 0;
     uint32_t* d_surv = nullptr;  // cull survivors
     size_t surv_cap = 0;
+    uint32_t* d_rest = nullptr;  // DgJobDev::rest (grown only for lazy jobs)
+    size_t rest_cap = 0;
     uint32_t* d_rec_of = nullptr;  // first triangle record of each survivor
     size_t rec_of_cap = 0;
     DgTriRec* d_trec = nullptr;

@@ -118,10 +118,10 @@ struct alignas(16) DgFrameDev {
     uint32_t small_max_px;  // this frame's small-triangle threshold (bounding-box pixels, <= 4096)
 };
 #define DG_FRAME_PERSPECTIVE 1u
-// The frame has at least as many triangles as pixels: its small triangles
-// (boxes of at most small_max_px pixels) get no light/halfway rows; the
-// resolve pass computes their vertices' vectors for the pixels they win
-// (DG_TRI_LAZY in the record's tie word).
+// The frame has at least as many triangles as pixels and a large light/halfway
+// table: its small unclipped triangles (boxes of at most small_max_px pixels) get
+// neither a triangle record nor light/halfway rows, only their small-list entry
+// (DG_LEAN in rec_of); the resolve pass shades the pixels they win from the mesh.
 #define DG_FRAME_LAZY 2u
 static_assert(sizeof(DgTexDev) == 48 && sizeof(DgMatDev) == 48, "descriptor sizes");
 // 1 if texel indices inside the map need neither 64-bit offsets nor a check of
@@ -191,10 +191,9 @@ struct DgEdges {
 // row's covered span can be estimated to within a few pixels (row_span).
 #define DG_EDGE_RCP 32u
 #define DG_EDGE_SPAN 64u
-// Set in a triangle record's tie word when its vertices have no light/halfway
-// rows (DG_FRAME_LAZY): shading computes them from the vertex positions, with
-// the same functions that fill the rows, so the values are identical.
-#define DG_TRI_LAZY 16u
+// Set in rec_of for a triangle without a record whose small-list entry is the
+// low 31 bits (DG_FRAME_LAZY; records of such jobs have numbers below 2^31).
+#define DG_LEAN 0x80000000u
 
 // One triangle (or one clip output of it) as the raster and shade passes read
 // it: twelve 16-byte words. Attribute fields hold the three vertices' values
@@ -291,7 +290,8 @@ inline uint32_t dg_item_log2(uint32_t item_units) {
 #define DG_CNT_TITEMX (11 * DG_CNT_LINE)  // further items of the transparent outputs
 #define DG_CNT_TSLOT (12 * DG_CNT_LINE)   // fragment nodes handed out (chunks of DG_FRAG_CHUNK)
 #define DG_CNT_CELLS (13 * DG_CNT_LINE)   // reached cells (jobs with split_below)
-#define DG_NCOUNTERS (14 * DG_CNT_LINE)   // words of the counter array
+#define DG_CNT_REST (14 * DG_CNT_LINE)    // entries of rest
+#define DG_NCOUNTERS (15 * DG_CNT_LINE)   // words of the counter array
 
 struct DgJobDev {
     const DgFrameDev* frames;
@@ -305,7 +305,8 @@ struct DgJobDev {
     uint32_t vrow_extra;    // rows after total_vtx available to clip vertices
     uint8_t* vmark;         // one byte per job vertex: needs light/halfway vectors (kept zero between jobs)
     uint32_t* surv;         // [total_tri] job-wide indices of the triangles that passed the cull pass
-    uint32_t* rec_of;       // [total_tri] first DgTriRec of each surviving triangle, or DG_NONE
+    uint32_t* rec_of;       // [total_tri] first DgTriRec of each surviving triangle, DG_LEAN | entry, or DG_NONE
+    uint32_t* rest;         // [total_tri] survivors that k_setup_lean leaves to k_setup_raster (jobs with lazy)
     DgTriRec* trec;
     // Per triangle record, (1/w_a, 1/w_b, 1/w_c, 0) of its three vertices' clip
     // w: written and read only for frames with DG_FRAME_PERSPECTIVE (null when
@@ -399,6 +400,7 @@ struct DgLaunchCfg {
     unsigned vertex_blocks;  // grid caps / sizes in 256-thread blocks
     unsigned cull_blocks;
     unsigned setup_blocks;
+    unsigned lean_blocks;
     unsigned queue_blocks;
     const DgInlineDesc* inl;  // host memory, read at launch; null: descriptors already on the device
     bool front;               // with inl: k_front in place of the vertex, cull and setup passes
@@ -422,6 +424,7 @@ struct DgLaunchCfg {
 #define DG_FRONT_MAX_TRI 131072u
 #endif
 #define DG_FRONT_THREADS 128u
+#define DG_LEAN_BLOCKS_PER_SM 6u  // one wave of k_setup_lean
 #define DG_CLIP_DEFER 512u  // k_setup_raster: clipped survivors a block sets up in its second pass
 // k_queue_raster's grid: 3 waves of its 4 resident blocks per SM. The passes'
 // work items are taken in a fixed strided order, so later waves even out

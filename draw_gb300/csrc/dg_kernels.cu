@@ -220,6 +220,11 @@ __global__ void __launch_bounds__(256) k_cull(const DgJobDev job) {
 // clipping, triangle records, bounding boxes and edge functions; tiny
 // triangles are rasterized by their warp, the others are queued
 // (scene/mod.rs:1029-1063, canvas.rs:585-681).
+// Whether a triangle with a box of px pixels goes to the small-triangle list.
+__device__ __forceinline__ bool small_listed(const DgFrameDev& fr, const RTri& tr, uint64_t px) {
+    return px <= fr.small_max_px && tr.xhi < 65536u && tr.yhi < 65536u && tr.xhi - tr.xlo < 255u &&
+           tr.yhi - tr.ylo < 255u && tr.frame < 65536u;
+}
 __device__ __forceinline__ void store_small(DgSmallRec* s, const RTri& tr) {
     float4* d = reinterpret_cast<float4*>(s);
     d[0] = make_float4(tr.ax, tr.bx, tr.cx, tr.ay);
@@ -246,7 +251,9 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
     }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
-    const unsigned long long ns64 = FRONT ? job.total_tri : __ldcg(job.cnt + DG_CNT_SURV);
+    // (in a lazy job, k_setup_lean has taken most survivors and listed the rest)
+    const uint32_t* list = job.lazy ? job.rest : job.surv;
+    const unsigned long long ns64 = FRONT ? job.total_tri : __ldcg(job.cnt + (job.lazy ? DG_CNT_REST : DG_CNT_SURV));
     const uint32_t nsurv = (uint32_t)(ns64 < job.total_tri ? ns64 : job.total_tri);
     // Pass 0 sets up the survivors, strided over the grid, but defers those that
     // need near/far clipping (up to DG_CLIP_DEFER per block) to pass 1, where the
@@ -268,7 +275,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                 i = valid ? s_clip_i[base + lane] : 0u;
                 g = valid ? s_clip_g[base + lane] : 0u;
             } else if (valid) {
-                g = FRONT ? i : __ldcg(job.surv + i);
+                g = FRONT ? i : __ldcg(list + i);
             }
             int nout = 0;
             uint32_t si = 0, t = 0, row0 = 0, nrows = 0;
@@ -326,9 +333,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                     clipped = true;
                     if (nout > 0 && P.nv > 3) nrows = (uint32_t)(P.nv - 3);  // light rows for the new vertices
                 }
-                // its vertices need light/halfway vectors for shading (in a DG_FRAME_LAZY
-                // frame an unclipped triangle is marked below, unless its record is lazy)
-                if (nout > 0 && (clipped || !(frame(sg.frame).flags & DG_FRAME_LAZY))) {
+                if (nout > 0) {  // its vertices need light/halfway vectors for shading
                     const uint32_t vv[3] = {sg.vtx_begin + tp.x, sg.vtx_begin + tp.y, sg.vtx_begin + tp.z};
                     for (int k = 0; k < 3; k++) job.vmark[vv[k]] = 1u;  // plain stores: every writer writes 1
                 }
@@ -396,14 +401,6 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                         boxed = true;
                         make_edges(tr.ax, tr.ay, tr.bx, tr.by, tr.cx, tr.cy, e);
                         const uint64_t px = (uint64_t)(tr.xhi - tr.xlo + 1u) * (uint64_t)(tr.yhi - tr.ylo + 1u);
-                        if ((fr.flags & DG_FRAME_LAZY) && !clipped) {
-                            if (rbase != DG_NONE && px <= fr.small_max_px) {
-                                e.tie |= DG_TRI_LAZY;  // no rows: shading computes the vertices' vectors
-                            } else {
-                                const uint32_t vv[3] = {sg.vtx_begin + tp.x, sg.vtx_begin + tp.y, sg.vtx_begin + tp.z};
-                                for (int k = 0; k < 3; k++) job.vmark[vv[k]] = 1u;
-                            }
-                        }
                         if (rbase != DG_NONE) {
                             float4* wout = (fr.flags & DG_FRAME_PERSPECTIVE) && job.trec_w
                                                ? job.trec_w + rbase + (uint32_t)rr
@@ -416,8 +413,7 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                         }
                         if (rbase == DG_NONE) {
                             inplace = true;
-                        } else if (px <= fr.small_max_px && tr.xhi < 65536u && tr.yhi < 65536u &&
-                                   tr.xhi - tr.xlo < 255u && tr.yhi - tr.ylo < 255u && tr.frame < 65536u) {
+                        } else if (small_listed(fr, tr, px)) {
                             small = true;
                         } else {
                             nu = (uint32_t)((px + DG_UNIT_PX - 1u) / DG_UNIT_PX);
@@ -577,6 +573,82 @@ __global__ void __launch_bounds__(256) k_setup_raster(const __grid_constant__ Dg
     DG_TL_WAITED(2);
     dev_setup<false>(job, job.nsegs, [&](uint32_t i) -> const DgSegDev& { return job.segs[i]; },
                      [&](uint32_t i) -> const DgFrameDev& { return job.frames[i]; });
+}
+
+// Setup of the small unclipped triangles of DG_FRAME_LAZY frames, before
+// k_setup_raster: their box and their small-list entry, and nothing else (no
+// edges, no record, no vertex marks); the other survivors go to the rest list.
+// Most triangles of such a frame win no pixel, so what shading needs is gathered
+// for the pixels instead. Bound by the gathers of the vertex records and by the
+// entries written; without the clip program and the record it runs at three times
+// the occupancy of k_setup_raster.
+__global__ void __launch_bounds__(256, 6) k_setup_lean(const __grid_constant__ DgJobDev job) {
+    wait_previous_kernel();
+    __shared__ uint32_t s_records;  // statistics, as in dev_setup
+    if (threadIdx.x == 0) s_records = 0u;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long ns64 = __ldcg(job.cnt + DG_CNT_SURV);
+    const uint32_t nsurv = (uint32_t)(ns64 < job.total_tri ? ns64 : job.total_tri);
+    for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < nsurv; base += gridDim.x * blockDim.x) {
+        uint32_t g = 0;
+        bool lean = false, rest = false, counted = false;
+        RTri tr;
+        const DgFrameDev* fr = job.frames;
+        if (base + lane < nsurv) {
+            g = __ldcg(job.surv + base + lane);
+            const DgSegDev& sg = job.segs[seg_of_tri(job, g)];
+            fr = job.frames + sg.frame;
+            const uint32_t t = g - sg.tri_begin;
+            float4 r[3];
+            triangle_vertices(job, sg, *fr, __ldg(sg.tri_pos + t), r);
+            const uint32_t m = __float_as_uint(r[0].w) & __float_as_uint(r[1].w) & __float_as_uint(r[2].w);
+            rest = !(fr->flags & DG_FRAME_LAZY) || (m & 0x3u) != 0x3u;
+            if (!rest) {
+                tr.ax = r[0].x; tr.ay = r[0].y;
+                tr.bx = r[1].x; tr.by = r[1].y;
+                tr.cx = r[2].x; tr.cy = r[2].y;
+                tr.da = r[0].z; tr.db = r[1].z; tr.dc = r[2].z;
+                tr.frame = sg.frame;
+                tr.seq = (sg.seq_base + t) << 2;
+                if (isnan(tr.ax) || isnan(tr.ay) || isnan(tr.bx) || isnan(tr.by) || isnan(tr.cx) || isnan(tr.cy)) {
+                    counted = true;  // every barycentric is NaN: nothing is covered
+                } else {
+                    bbox_axis(tr.ax, tr.bx, tr.cx, fr->width, tr.xlo, tr.xhi);
+                    bbox_axis(tr.ay, tr.by, tr.cy, fr->height, tr.ylo, tr.yhi);
+                    lean = small_listed(*fr, tr, (uint64_t)(tr.xhi - tr.xlo + 1u) * (tr.yhi - tr.ylo + 1u));
+                    rest = !lean;
+                }
+            }
+        }
+        const unsigned lmask = __ballot_sync(FULL, lean), rmask = __ballot_sync(FULL, rest);
+        unsigned long long lold = 0, rold = 0;
+        if (lane == 0u) {
+            if (lmask) lold = atomicAdd(job.cnt + DG_CNT_SMALL, (unsigned long long)__popc(lmask));
+            if (rmask) rold = atomicAdd(job.cnt + DG_CNT_REST, (unsigned long long)__popc(rmask));
+        }
+        const unsigned below = (1u << lane) - 1u;
+        const uint64_t slot = __shfl_sync(FULL, lold, 0) + __popc(lmask & below);
+        uint64_t rpos = __shfl_sync(FULL, rold, 0) + __popc(rmask & below);
+        if (lean && slot >= job.small_cap) {  // list full
+            lean = false;
+            rest = true;
+            rpos = atomicAdd(job.cnt + DG_CNT_REST, 1ull);
+        }
+        if (rest) job.rest[rpos] = g;  // each survivor once: at most total_tri
+        if (lean) {
+            store_small(job.small + slot, tr);
+            job.rec_of[g] = DG_LEAN | (uint32_t)slot;
+            if (fr->cells != nullptr)  // the box's 32x32 cells, as in dev_setup
+                for (uint32_t cy = tr.ylo >> 5; cy <= tr.yhi >> 5; cy++)
+                    for (uint32_t cx = tr.xlo >> 5; cx <= tr.xhi >> 5; cx++)
+                        fr->cells[cy * fr->tiles_x + cx] = fr->epoch;
+        }
+        const uint32_t n = (uint32_t)__popc(__ballot_sync(FULL, lean || counted));
+        if (lane == 0u && n) atomicAdd(&s_records, n);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_records) atomicAdd(job.cnt + DG_CNT_TREC, (unsigned long long)s_records);
 }
 
 // The front of a small job as one kernel instead of three: vertex, cull and setup
@@ -997,8 +1069,9 @@ __device__ __forceinline__ void clear_tile(const DgFrameDev& fr, uint32_t tx, ui
 // One tile of the resolve pass (block-uniform; the tables of resolve_prologue
 // must be in place). EXT: the job uses an extension mode (perspective-correct
 // interpolation or bilinear fetch); false compiles the reference's shading only.
-// LAZY: a frame of the job has DG_FRAME_LAZY (records of small triangles carry
-// no light rows).
+// LAZY: a frame of the job has DG_FRAME_LAZY (its small triangles have no
+// records); the resolve kernels then run at three blocks per SM, since the mesh's
+// attributes and the vertices' vectors need registers.
 template <uint32_t TH, bool EXT, bool LAZY>
 __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const DgFrameDev& fr, const uint32_t tx,
                                                  const uint32_t ty, const float* inv255, const DgTexDev* stex) {
@@ -1051,7 +1124,9 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const DgFr
                 if (t < sg.ntri) val[j] = __ldg(job.rec_of + sg.tri_begin + t);
             }
             const uint32_t o = (uint32_t)key[j] & 3u;
-            if (val[j] != DG_NONE && val[j] + o < job.trec_cap) {  // trec_cap <= 2^32 - 16
+            if (LAZY && val[j] != DG_NONE && (val[j] & DG_LEAN)) {
+                fr.vis[i] = DG_VIS_EMPTY;  // (its one output)
+            } else if (val[j] != DG_NONE && val[j] + o < job.trec_cap) {  // trec_cap <= 2^32 - 16
                 val[j] += o;
                 fr.vis[i] = DG_VIS_EMPTY;
             } else {
@@ -1095,8 +1170,11 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const DgFr
         const uint32_t px = tx * DG_TILE_W + (pe & 31u), py = ty * TH + (pe >> 5);
         float d = 0.0f;
         int errc;
-        const float4* wp = EXT && (fr.flags & DG_FRAME_PERSPECTIVE) && job.trec_w ? job.trec_w + s_val[k] : nullptr;
-        uint32_t c = shade_from_record<EXT, LAZY>(job, fr, job.trec + s_val[k], px, py, inv255, stex, d, errc, wp);
+        const uint32_t rec = s_val[k];
+        const DgSmallRec* lean = LAZY && (rec & DG_LEAN) ? job.small + (rec & ~DG_LEAN) : nullptr;
+        const float4* wp =
+            EXT && (fr.flags & DG_FRAME_PERSPECTIVE) && job.trec_w && !lean ? job.trec_w + rec : nullptr;
+        uint32_t c = shade_from_record<EXT, LAZY>(job, fr, job.trec + rec, px, py, inv255, stex, d, errc, wp, lean);
         if (errc != DG_OK) {
             c = AZUL_BB;
             errors |= 1u << errc;
@@ -1118,7 +1196,7 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const DgFr
 __device__ __forceinline__ bool resolve_early(const DgJobDev& job) { return job.ntt == 0u && job.total_tri != 0u; }
 
 template <uint32_t TH, bool EXT, bool LAZY>
-__global__ void __launch_bounds__(256, 4) k_resolve(const __grid_constant__ DgJobDev job) {
+__global__ void __launch_bounds__(256, LAZY ? 3 : 4) k_resolve(const __grid_constant__ DgJobDev job) {
     DG_TL_BLOCK(4);  // tiles cleared before the wait record no wait
     __shared__ float inv255[256];
     __shared__ DgTexDev stex[DG_SMEM_TEX];
@@ -1148,7 +1226,7 @@ __global__ void __launch_bounds__(256, 4) k_resolve(const __grid_constant__ DgJo
 // 1283x717 field that covers 17% of the frame: 53.4 us whole, 46.8 us by this
 // kernel; strips of more cells lose (ten frames of 500 reached cells 83 -> 86 us).
 template <bool EXT, bool LAZY>
-__global__ void __launch_bounds__(256, 4) k_resolve_split(const __grid_constant__ DgJobDev job) {
+__global__ void __launch_bounds__(256, LAZY ? 3 : 4) k_resolve_split(const __grid_constant__ DgJobDev job) {
     DG_TL_BLOCK(4);
     __shared__ float inv255[256];
     __shared__ DgTexDev stex[DG_SMEM_TEX];
@@ -1255,6 +1333,10 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else if (job.total_tri) {
         NvtxRange r("k_setup_raster");
+        if (job.lazy) {
+            const unsigned lb = cfg.lean_blocks < 1u ? 1u : cfg.lean_blocks;
+            if ((e = launch_dependent(k_setup_lean, grid_for(job.total_tri, lb), 256, job, s)) != cudaSuccess) return e;
+        }
         const unsigned sb = cfg.setup_blocks < 1u ? 1u : cfg.setup_blocks;
         if ((e = launch_dependent(k_setup_raster, grid_for(job.total_tri, sb), 256, job, s)) != cudaSuccess) return e;
     }

@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(256, DG_TRASTER_BLOCKS_PER_SM) k_traster(const
             float d;
             int errc;
             const float4* wp = EXT && (fr->flags & DG_FRAME_PERSPECTIVE) && job.ttrec_w ? job.ttrec_w + rec : nullptr;
-            const uint32_t c = shade_from_record<EXT, false>(job, *fr, job.ttrec + rec, x, y, inv255, stex, d, errc, wp);
+            const uint32_t c = shade_from_record<EXT, false>(job, *fr, job.ttrec + rec, x, y, inv255, stex, d, errc, wp, nullptr);
             if (errc != DG_OK) atomicOr(job.err, 1u << errc);
             link_fragment(job.fnode, job.fhead + pix, slot, key, c, __ldcg(job.talpha + rec));
         }
