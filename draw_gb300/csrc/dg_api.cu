@@ -475,7 +475,7 @@ uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L
     const size_t vmask = cap_after(s.vmask_cap, s.d_vmask, std::max<uint64_t>(V, 1));
     const size_t vrec = cap_after(s.vrec_cap, s.d_vrec, std::max<uint64_t>(V, 1));
     const size_t vshade = cap_after(s.vshade_cap, s.d_vshade, (V + dg_vrow_extra(T)) * L * 2);
-    const size_t vmark = cap_after(s.vmark_cap, s.d_vmark, std::max<uint64_t>(V, 1));
+    const size_t vmark = cap_after(s.vmark_cap, s.d_vmark, (V + 512) & ~511ull);
     const size_t q = cap_after(s.queue_cap, s.d_queue, queue_records(T));
     const size_t sm = cap_after(s.small_cap, s.d_small, queue_records(T));
     const size_t qb = cap_after(s.items_cap, s.d_items, dg_items_cap(q));
@@ -713,7 +713,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
             if (e) return e;
         }
     }
-    const size_t want_mark = std::max<uint64_t>(total_vtx, 1);
+    const size_t want_mark = (total_vtx + 512) & ~511ull;  // read in groups of 512
     if (S.vmark_cap < want_mark) {
         e = grow(S, &S.d_vmark, &S.vmark_cap, want_mark);
         if (e) return e;

@@ -395,7 +395,9 @@ __device__ __forceinline__ void dev_setup(const DgJobDev& job, uint32_t nsegs, S
                     }
                     bool nan = isnan(tr.ax) || isnan(tr.ay) || isnan(tr.bx) || isnan(tr.by) || isnan(tr.cx) ||
                                isnan(tr.cy);
-                    if (!nan) {  // any NaN centre makes every barycentric NaN: nothing is covered
+                    // any NaN centre makes every barycentric NaN: nothing is covered (unclipped
+                    // triangles without area were dropped before)
+                    if (!nan && !(clipped && covers_nothing(tr.ax, tr.ay, tr.bx, tr.by, tr.cx, tr.cy, fr.width, fr.height))) {
                         bbox_axis(tr.ax, tr.bx, tr.cx, fr.width, tr.xlo, tr.xhi);
                         bbox_axis(tr.ay, tr.by, tr.cy, fr.height, tr.ylo, tr.yhi);
                         boxed = true;
@@ -702,14 +704,16 @@ __device__ __forceinline__ SmallTri load_small(const DgSmallRec* s) {
 #define DG_SMALL_STRIDE 7
 #define DG_SMALL_WINDOW 512u  // covered pixels listed at a time
 // Rasterizes entries first .. first + 31 of the small-triangle list. Each lane
-// tests its box's pixels one after another into a mask (edges in registers, one
-// comparison per edge); the covered pixels of all 32 are then listed together
+// tests its box's pixels one after another into a mask (edge values in registers,
+// one addition per edge and pixel); the covered pixels of all 32 are then listed together
 // and finished one per lane, so that the divisions and the keyed minimum run on
 // full warps (about a fifth of the box pixels are covered, unevenly). Measured
 // for the queue pass on 10M micro triangles and on 32 small frames: 306 and 53
 // us; with the pixels of all boxes numbered together and one per lane, 393 and
 // 57; a lane finishing its own pixels, triangles ordered by box size, 411 and 70
-// (before covers_nothing).
+// (before covers_nothing). With the edge values evaluated anew at each pixel, clip
+// outputs without area listed too (57 us of it), plain divisions (bary_fast) and a
+// load of the vertex marks per 32 (40 us), the micro frame took 264; now 170.
 __device__ __forceinline__ void raster_small_chunk(const DgJobDev& job, uint32_t first, uint32_t nsmall, float4* st,
                                                    uint16_t* list) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -728,26 +732,60 @@ __device__ __forceinline__ void raster_small_chunk(const DgJobDev& job, uint32_t
         d[4] = make_float4(t.e.den[0], t.e.den[1], t.e.den[2], __uint_as_float(t.seq));
         d[5] = make_float4(t.da, t.db, t.dc, 0.0f);
         if (!whole) {
-            // covered_signs as one comparison: the edge values are integer-valued (or
-            // infinite), so "> 0, or 0 with the tie bit" is "> 0" or "> -1/2"
-            const float t0 = (t.e.tie & 1u) ? -0.5f : 0.0f, t1 = (t.e.tie & 2u) ? -0.5f : 0.0f,
-                        t2 = (t.e.tie & 4u) ? -0.5f : 0.0f;
-            const float xlo = (float)t.x0, xend = (float)(t.x0 + t.w);
-            float xf = xlo, yf = (float)t.y0;
-            uint32_t m[2] = {0u, 0u};
+            // covered_signs as a sign: the edge values are integer-valued (or infinite),
+            // so "> 0, or 0 with the tie bit" is "> -1/2" or "> 1/2".
+            const float t0 = (t.e.tie & 1u) ? 0.5f : -0.5f, t1 = (t.e.tie & 2u) ? 0.5f : -0.5f,
+                        t2 = (t.e.tie & 4u) ? 0.5f : -0.5f;
+            // When no step of an edge value rounds anywhere in the box, moving a pixel
+            // adds exactly A and moving a row exactly B: |C|, |D| < 2^23 and |A| x + |B| y
+            // < 2^22 keep the sums integers below 2^24, and values below 2^22 in the box
+            // take the half exactly.
+            const float bx = (float)(t.x0 + t.w), by = (float)(t.y0 + t.h), bw = (float)t.w, bh = (float)t.h;
+            const float xf = (float)t.x0, yf = (float)t.y0;
+            float f0 = edge_eval(t.e, 0, xf, yf), f1 = edge_eval(t.e, 1, xf, yf), f2 = edge_eval(t.e, 2, xf, yf);
+            const float fm[3] = {fabsf(f0), fabsf(f1), fabsf(f2)};
+            bool exact = true;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const float aA = fabsf(t.e.A[k]), aB = fabsf(t.e.B[k]);
+                exact = exact && fmaxf(fabsf(t.e.C[k]), fabsf(t.e.D[k])) < 0x1p23f && aA * bx + aB * by < 0x1p22f &&
+                        fm[k] + aA * bw + aB * bh < 0x1p22f;
+            }
+            f0 += t0;
+            f1 += t1;
+            f2 += t2;
+            const float wm = (float)(t.w - 1u);  // from a row's last pixel to the next row's first
+            const float w0 = t.e.B[0] - wm * t.e.A[0], w1 = t.e.B[1] - wm * t.e.A[1], w2 = t.e.B[2] - wm * t.e.A[2];
+            uint32_t m[2] = {0u, 0u}, c = 0;
 #pragma unroll
             for (int half = 0; half < 2; half++) {
-                const uint32_t end = n < 32u ? n : half == 0 ? 32u : n;
-                for (uint32_t k = 32u * half; k < end; k++) {
-                    const bool in = (edge_eval(t.e, 0, xf, yf) > t0) & (edge_eval(t.e, 1, xf, yf) > t1) &
-                                    (edge_eval(t.e, 2, xf, yf) > t2);
-                    m[half] |= (in ? 1u : 0u) << (k & 31u);
-                    xf += 1.0f;
-                    if (xf == xend) {
-                        xf = xlo;
-                        yf += 1.0f;
+                const uint32_t begin = 32u * half, end = n < begin + 32u ? n : begin + 32u;
+                uint32_t out = 0;  // outside bits, the first pixel's highest
+                for (uint32_t k = begin; k < end; k++) {
+                    out = __funnelshift_l(__float_as_uint(f0) | __float_as_uint(f1) | __float_as_uint(f2), out, 1u);
+                    const bool wrap = ++c == t.w;
+                    c = wrap ? 0u : c;
+                    f0 += wrap ? w0 : t.e.A[0];
+                    f1 += wrap ? w1 : t.e.A[1];
+                    f2 += wrap ? w2 : t.e.A[2];
+                }
+                if (end > begin) m[half] = __brev(~out) >> (32u - (end - begin));
+            }
+            if (!exact) {  // the edge values as the reference evaluates them
+                float x = xf, y = yf;
+                uint64_t mm = 0;
+                for (uint32_t k = 0; k < n; k++) {
+                    const bool in = (edge_eval(t.e, 0, x, y) > -t0) & (edge_eval(t.e, 1, x, y) > -t1) &
+                                    (edge_eval(t.e, 2, x, y) > -t2);
+                    mm |= (in ? 1ull : 0ull) << k;
+                    x += 1.0f;
+                    if (x == bx) {
+                        x = xf;
+                        y += 1.0f;
                     }
                 }
+                m[0] = (uint32_t)mm;
+                m[1] = (uint32_t)(mm >> 32);
             }
             mask = ((uint64_t)m[1] << 32) | m[0];
         }
@@ -782,9 +820,9 @@ __device__ __forceinline__ void raster_small_chunk(const DgJobDev& job, uint32_t
             const uint32_t x = (xy & 0xFFFFu) + (k - dy * __float_as_uint(box.y)), y = (xy >> 16) + dy;
             const float xf = (float)x, yf = (float)y;
             const DgFrameDev& fr = job.frames[__float_as_uint(box.w)];
-            const float al = fD(edge_eval(e, 0, xf, yf), den.x);
-            const float be = fD(edge_eval(e, 1, xf, yf), den.y);
-            const float ga = fD(edge_eval(e, 2, xf, yf), den.z);
+            const float al = bary_fast(edge_eval(e, 0, xf, yf), den.x);
+            const float be = bary_fast(edge_eval(e, 1, xf, yf), den.y);
+            const float ga = bary_fast(edge_eval(e, 2, xf, yf), den.z);
             const float depth = interp(al, be, ga, dd.x, dd.y, dd.z);
             if (depth < fr.clear_depth)
                 atomicMin(reinterpret_cast<unsigned long long*>(fr.vis) + (y * fr.width + x),
@@ -815,11 +853,26 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
     // Prologue: light/halfway vectors of the vertices the setup pass marked, 32
     // vertices per warp; the marks are cleared for the next job.
     const uint32_t ngroups = (job.total_vtx + 31u) >> 5;
-    for (uint32_t w = warp; w < ngroups; w += nwarps) {
+    auto shade_group = [&](uint32_t w) {
         const uint32_t v = (w << 5) + lane;
         if (v < job.total_vtx && __ldcg(job.vmark + v)) {
             shade_vertex(job, v);
             job.vmark[v] = 0u;
+        }
+    };
+    if (ngroups <= 4u * nwarps) {
+        for (uint32_t w = warp; w < ngroups; w += nwarps) shade_group(w);
+    } else {
+        // Many vertices: 512 marks per load first (a load per 32 of 9M vertices was a chain
+        // of 19 per warp, 40 us of the queue pass).
+        for (uint32_t w = warp; w < (ngroups + 15u) >> 4; w += nwarps) {
+            const uint4 m = __ldcg(reinterpret_cast<const uint4*>(job.vmark) + (w << 5) + lane);
+            unsigned any = __ballot_sync(FULL, (m.x | m.y | m.z | m.w) != 0u);
+            while (any) {  // lanes 2 g and 2 g + 1 hold the marks of group g
+                const uint32_t g = ((uint32_t)__ffs(any) - 1u) >> 1;
+                any &= ~(3u << (2u * g));
+                shade_group((w << 4) + g);
+            }
         }
     }
     const unsigned long long cnt = __ldcg(job.cnt + DG_CNT_QUEUE);
