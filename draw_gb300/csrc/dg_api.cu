@@ -643,11 +643,11 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     if (e) return e;
     // A small job: descriptors as a kernel parameter, and up to DG_FRONT_MAX_TRI
     // triangles the one-kernel front, which needs no sign masks and no survivor list.
-    B.inline_desc = B.inline_ok && n == 1 && segs.size() <= DG_INLINE_SEGS && total_vtx > 0;
+    B.inline_desc = B.inline_ok && total_vtx > 0 && n <= DgInlineLarge::kFrames && segs.size() <= DgInlineLarge::kSegs;
     B.cfg.front = B.inline_desc && total_tri > 0 && total_tri <= DG_FRONT_MAX_TRI;
     if (B.cfg.front && any_lazy) {  // the one-kernel front writes full records
         any_lazy = false;
-        frames[0].flags &= ~DG_FRAME_LAZY;
+        for (DgFrameDev& f : frames) f.flags &= ~DG_FRAME_LAZY;
     }
     if (any_lazy) {
         e = grow(S, &S.d_rest, &S.rest_cap, total_tri);
@@ -871,12 +871,24 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
     // A small job's descriptors go to the device as a kernel parameter (k_vertex
     // writes them to the staging buffer); larger ones are copied.
     DgInlineDesc inl;
-    if (B.inline_desc) {
-        std::memset(&inl, 0, sizeof(inl));
-        inl.frame = B.frames[0];
-        for (size_t i = 0; i < B.segs.size(); i++) inl.segs[i] = B.segs[i];
-        inl.nsegs = (uint32_t)B.segs.size();
+    DgInlineBatch inl_batch;
+    DgInlineLarge inl_large;
+    auto fits = [&](auto& d) { return n <= d.kFrames && B.segs.size() <= d.kSegs; };
+    auto fill = [&](auto& d) {
+        std::copy(B.frames.begin(), B.frames.end(), d.frames);
+        std::copy(B.segs.begin(), B.segs.end(), d.segs);
+        d.nframes = (uint32_t)B.frames.size();
+        d.nsegs = (uint32_t)B.segs.size();
+    };
+    if (B.inline_desc && fits(inl)) {
+        fill(inl);
         B.cfg.inl = &inl;
+    } else if (B.inline_desc && fits(inl_batch)) {
+        fill(inl_batch);
+        B.cfg.inl_batch = &inl_batch;
+    } else if (B.inline_desc) {
+        fill(inl_large);
+        B.cfg.inl_large = &inl_large;
     } else {
         std::memcpy(S.h_stage[k], B.frames.data(), B.fbytes);
         std::memcpy((uint8_t*)S.h_stage[k] + B.fbytes, B.segs.data(), B.sbytes);

@@ -383,17 +383,25 @@ struct DgTransparentPlan {
 // leave one chunk partly used.
 constexpr uint64_t dg_frag_nodes(uint64_t n, unsigned blocks) { return n + (uint64_t)blocks * 8u * DG_FRAG_CHUNK; }
 
-// The descriptors of a small job (one frame, at most DG_INLINE_SEGS segments)
-// travel as a kernel parameter of k_vertex instead of a host-to-device copy:
-// k_vertex reads them from its parameter and writes them to job.frames and
-// job.segs, where the later kernels of the job read them.
-#define DG_INLINE_SEGS 4
-struct alignas(16) DgInlineDesc {
-    DgFrameDev frame;
-    DgSegDev segs[DG_INLINE_SEGS];
-    uint32_t nsegs;  // 0: the descriptors were copied to the device by the host
-    uint32_t pad[3];
+// The descriptors of a small job travel as a kernel parameter of its first kernel
+// instead of a host-to-device copy: that kernel reads them from its parameter and
+// writes them to job.frames and job.segs, where the later kernels of the job read
+// them. A copy before the first kernel keeps it from starting under the previous
+// job's last one: batches of 2, 10 and 28 frames, one object each, took 33.3, 73.4
+// and 92.0 us with it and take 20.7, 66.0 and 81.9 us without (the first with
+// k_front as well). A launch copies its whole parameter (at most 32,764 bytes), so
+// there are three sizes: a batch of 10 took 0.5 us more with twice the room.
+template <uint32_t F, uint32_t S>
+struct alignas(16) DgInlineDescT {
+    static constexpr uint32_t kFrames = F, kSegs = S;
+    DgFrameDev frames[F];
+    DgSegDev segs[S];
+    uint32_t nframes, nsegs;  // nsegs 0: the descriptors were copied to the device by the host
+    uint32_t pad[2];
 };
+using DgInlineDesc = DgInlineDescT<1, 4>;
+using DgInlineBatch = DgInlineDescT<16, 24>;
+using DgInlineLarge = DgInlineDescT<48, 72>;
 
 // Host-side launchers (dg_kernels.cu).
 struct DgLaunchCfg {
@@ -402,8 +410,11 @@ struct DgLaunchCfg {
     unsigned setup_blocks;
     unsigned lean_blocks;
     unsigned queue_blocks;
-    const DgInlineDesc* inl;  // host memory, read at launch; null: descriptors already on the device
-    bool front;               // with inl: k_front in place of the vertex, cull and setup passes
+    // Descriptors in host memory, read at launch; all null: already on the device.
+    const DgInlineDesc* inl;
+    const DgInlineBatch* inl_batch;
+    const DgInlineLarge* inl_large;
+    bool front;  // with one of them: k_front in place of the vertex, cull and setup passes
     DgTransparentPlan tplan;
 };
 // k_vertex's grid cap: its resident blocks (launch bounds 256 x 8), one wave
@@ -411,13 +422,14 @@ struct DgLaunchCfg {
 // headline frame 88.8 -> 87.8 us, the stress frame's vertex pass 64 -> 59 us).
 #define DG_VERTEX_BLOCKS_PER_SM 8u
 #define DG_SETUP_BLOCKS_PER_SM 4u
-// Jobs of one frame whose descriptors travel inline and of at most this many
-// triangles take k_front instead of the vertex, cull and setup passes: it saves
-// two launches and their dependent loads, and computes each vertex once per
-// triangle. Measured, three passes against k_front: 200 triangles 23.6 / 20.1 us
-// a frame, 4,800 38.7 / 33.4, 60,000 34.9 / 31.0, 150,000 38.1 / 37.8, 300,000
-// 53.8 / 55.4, a million 93.8 / 111 us. Blocks of 128 threads: 64 and 256 measured
-// the same or up to 2 us slower.
+// Jobs whose descriptors travel inline and of at most this many triangles take
+// k_front instead of the vertex, cull and setup passes: it saves two launches and
+// their dependent loads, and computes each vertex once per triangle. Measured,
+// three passes against k_front: one frame of 200 triangles 23.6 / 20.1 us, 4,800
+// 38.7 / 33.4, 60,000 34.9 / 31.0, 160,000 49.3 / 49.2, 200,000 35.8 / 37.8, a
+// million 93.8 / 111; batches of 156,000 68.0 / 65.9, 169,000 67.9 / 69.1, 192,000
+// 46.7 / 44.9, 280,000 81.8 / 82.7. Blocks of 128 threads: 64 and 256 measured the
+// same or up to 2 us slower.
 #if DG_TIMELINE
 #define DG_FRONT_MAX_TRI 0u  // the timeline shows every pass as a kernel of its own
 #else

@@ -107,35 +107,37 @@ __device__ __forceinline__ void dev_vertex(const DgJobDev& job, uint32_t nsegs, 
 // A job's first kernel: zeroes the counters of the slot's next job (this job's
 // were zeroed by the job before it) and, for a small job, writes the descriptors
 // of its parameter `in` to job.frames and job.segs.
-__device__ __forceinline__ void begin_job(const DgJobDev& job, const DgInlineDesc& in) {
-    if (blockIdx.x != 0) return;
-    if (job.cnt_next)
+template <class IN>
+__device__ __forceinline__ void begin_job(const DgJobDev& job, const IN& in) {
+    if (job.cnt_next && blockIdx.x == 0)
         for (uint32_t i = threadIdx.x; i < DG_NCOUNTERS; i += blockDim.x) job.cnt_next[i] = 0ull;
     if (in.nsegs) {
         constexpr uint32_t fw = sizeof(DgFrameDev) / 8, sw = sizeof(DgSegDev) / 8;
         static_assert(sizeof(DgFrameDev) % 8 == 0 && sizeof(DgSegDev) % 8 == 0, "8-byte words");
         uint2* fd = reinterpret_cast<uint2*>(const_cast<DgFrameDev*>(job.frames));
         uint2* sd = reinterpret_cast<uint2*>(const_cast<DgSegDev*>(job.segs));
-        const uint2* fs = reinterpret_cast<const uint2*>(&in.frame);
+        const uint2* fs = reinterpret_cast<const uint2*>(in.frames);
         const uint2* ss = reinterpret_cast<const uint2*>(in.segs);
-        for (uint32_t i = threadIdx.x; i < fw + in.nsegs * sw; i += blockDim.x) {
-            if (i < fw)
+        const uint32_t nf = in.nframes * fw, stride = gridDim.x * blockDim.x;
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nf + in.nsegs * sw; i += stride) {
+            if (i < nf)
                 fd[i] = fs[i];
             else
-                sd[i - fw] = ss[i - fw];
+                sd[i - nf] = ss[i - nf];
         }
     }
 }
 
+template <class IN>
 __global__ void __launch_bounds__(256, 8) k_vertex(const __grid_constant__ DgJobDev job,
-                                                   const __grid_constant__ DgInlineDesc in) {
+                                                   const __grid_constant__ IN in) {
     DG_TL_BLOCK(0);
     allow_next_kernel();
     DG_TL_WAITED(0);  // the first kernel of a job waits on nothing (a stream-ordered launch)
     begin_job(job, in);
     if (in.nsegs)
         dev_vertex<true>(job, in.nsegs, [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; },
-                   [&](uint32_t) -> const DgFrameDev& { return in.frame; });
+                   [&](uint32_t i) -> const DgFrameDev& { return in.frames[IN::kFrames == 1u ? 0u : i]; });
     else
         dev_vertex<true>(job, job.nsegs, [&](uint32_t i) -> const DgSegDev& { return job.segs[i]; },
                    [&](uint32_t i) -> const DgFrameDev& { return job.frames[i]; });
@@ -658,14 +660,15 @@ __global__ void __launch_bounds__(256, 6) k_setup_lean(const __grid_constant__ D
 // dependent loads each. A thread computes its triangle's three vertices itself
 // (about three times the vertex arithmetic of k_vertex); the vertex records that
 // the transparent pass and record-less pixels read are written at the end.
+template <class IN>
 __global__ void __launch_bounds__(DG_FRONT_THREADS) k_front(const __grid_constant__ DgJobDev job,
-                                                            const __grid_constant__ DgInlineDesc in) {
+                                                            const __grid_constant__ IN in) {
     DG_TL_BLOCK(2);
     allow_next_kernel();
     DG_TL_WAITED(2);
     begin_job(job, in);
     auto seg = [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; };
-    auto frame = [&](uint32_t) -> const DgFrameDev& { return in.frame; };
+    auto frame = [&](uint32_t i) -> const DgFrameDev& { return in.frames[IN::kFrames == 1u ? 0u : i]; };
     dev_setup<true>(job, in.nsegs, seg, frame);
     dev_vertex<false>(job, in.nsegs, seg, frame);
 }
@@ -1364,12 +1367,22 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     auto mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s) : cudaSuccess; };
     if ((e = mark(0)) != cudaSuccess) return e;
     DgInlineDesc none;
-    if (!cfg.inl) none.nsegs = 0;
-    const bool front = cfg.front && cfg.inl && job.total_vtx && job.total_tri;
+    none.nsegs = 0;
+    // calls f with the descriptors of the job's first kernel
+    auto with_inline = [&](auto f) {
+        if (cfg.inl_large)
+            f(*cfg.inl_large);
+        else if (cfg.inl_batch)
+            f(*cfg.inl_batch);
+        else
+            f(cfg.inl ? *cfg.inl : none);
+    };
+    const bool front =
+        cfg.front && (cfg.inl || cfg.inl_batch || cfg.inl_large) && job.total_vtx && job.total_tri;
     if (job.total_vtx && !front) {
         NvtxRange r("k_vertex");
         const unsigned vb = cfg.vertex_blocks < 1u ? 1u : cfg.vertex_blocks;
-        k_vertex<<<grid_for(job.total_vtx, vb), 256, 0, s>>>(job, cfg.inl ? *cfg.inl : none);
+        with_inline([&](const auto& in) { k_vertex<<<grid_for(job.total_vtx, vb), 256, 0, s>>>(job, in); });
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if ((e = mark(1)) != cudaSuccess) return e;
@@ -1382,7 +1395,7 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     if (front) {
         NvtxRange r("k_front");
         const uint32_t blocks = (job.total_tri + DG_FRONT_THREADS - 1u) / DG_FRONT_THREADS;
-        k_front<<<blocks, DG_FRONT_THREADS, 0, s>>>(job, *cfg.inl);
+        with_inline([&](const auto& in) { k_front<<<blocks, DG_FRONT_THREADS, 0, s>>>(job, in); });
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else if (job.total_tri) {
         NvtxRange r("k_setup_raster");

@@ -1,8 +1,10 @@
 """The one-kernel front of small jobs (vertex, cull and setup of at most 131,072
-triangles of one frame) against the three separate passes, which the same scene
-takes as part of a two-frame batch: both frames bit-identical, the statistics
-equal, and equal to the CPU oracle. At the sizes where the front's blocks and its
-limit end, on clipped geometry, and with several objects per frame."""
+triangles) against the three separate passes, which the same scene takes as part
+of a captured batch: frames bit-identical, and equal to the CPU oracle, and the
+statistics of a batch of two the sum of theirs. At the sizes where the front's
+blocks and its limit end, on clipped geometry, and with several objects per frame;
+and the descriptors that travel with the first kernel at the numbers of frames and
+objects where their room ends."""
 import numpy as np
 import pytest
 
@@ -61,6 +63,45 @@ def test_front_equals_separate_passes(name, gpu_ctx, oracle_lib):
     assert p.ok, f"{describe(p)}; {first_mismatch(ref, alone)}"
     assert np.array_equal(alone[0], batched[0])
     assert np.array_equal(alone[1].view(np.uint32), batched[1].view(np.uint32))
-    assert stats["launches"] == (3 if desc.n_tris <= 131072 else 5) and both["launches"] == 5
+    assert stats["launches"] == (3 if desc.n_tris <= 131072 else 5)
+    assert both["launches"] == (3 if desc.n_tris + cases.tie_rule_scene().n_tris <= 131072 else 5)
     for k in keys[:-1]:
         assert stats[k] + other[k] == both[k], (k, stats[k], other[k], both[k])
+    graph = gpu_ctx.batch([a.scene, b.scene], [a.canvas, b.canvas])  # the separate passes
+    try:
+        graph.render()
+        replayed = a.canvas.read()
+    finally:
+        graph.close()
+    assert np.array_equal(alone[0], replayed[0])
+    assert np.array_equal(alone[1].view(np.uint32), replayed[1].view(np.uint32))
+
+
+def _several(objects, n):
+    """A frame of several objects, another one for each n."""
+    parts = []
+    for k in range(objects):
+        c, s = np.cos(0.7 * k + n), np.sin(1.1 * k + n)
+        z = -0.3 * k
+        parts.append(cases._obj([[c - 2, s - 2, z], [c + 2, s - 2, z], [c, s + 2, z + 0.5 * c]], [[0, 1, 2]],
+                                [cases._mat(0)]))
+    return cases.flat_scene(parts, width=48 + n % 5, height=40 + n % 3)
+
+
+# frames, objects per frame: one frame of up to 4 objects, 16 frames with 24 objects in all, 48 with 72, more
+@pytest.mark.parametrize("frames,objects,tris", [(1, 4, 1), (1, 5, 1), (1, 24, 1), (1, 25, 1), (1, 72, 1), (1, 73, 1),
+                                                 (2, 12, 1), (2, 13, 1), (16, 1, 1), (17, 1, 1), (48, 1, 1), (49, 1, 1),
+                                                 (3, 1, 70_000), (13, 1, 10_000)])
+def test_descriptors_with_the_first_kernel(frames, objects, tris, gpu_ctx, oracle_lib):
+    from draw_gb300 import renderer
+
+    descs = [_several(objects, n) if tris == 1 else _triangles(tris + n) for n in range(frames)]
+    built = [renderer.build_scene(d, gpu_ctx) for d in descs]
+    for _ in range(2):
+        gpu_ctx.render_batch([b.scene for b in built], [b.canvas for b in built])
+    small = frames <= 48 and frames * objects <= 72 and sum(d.n_tris for d in descs) <= 131072
+    assert gpu_ctx.last_stats()["launches"] == (3 if small else 5)
+    for d, b in zip(descs, built):
+        ref, got = oracle_render(d), (*b.canvas.read(), 0)
+        p = compare(ref, got, d.clear_depth)
+        assert p.ok, f"{d.name}: {describe(p)}; {first_mismatch(ref, got)}"
