@@ -199,7 +199,7 @@ struct DgEdges {
 // it: twelve 16-byte words. Attribute fields hold the three vertices' values
 // in x, y, z (clip outputs: the values VertexAttributes arithmetic gives the
 // new vertices, canvas.rs:242-291); the w slots carry the triangle's material.
-struct alignas(16) DgTriRec {
+struct alignas(32) DgTriRec {
     DgEdges e;                    // words 0-3
     float da, db, dc, ka_x;       // word 4: vertex depths (eye distances)
     float u[3], ka_y;             // word 5: texture coordinates

@@ -916,7 +916,7 @@ __device__ __forceinline__ void dev_queue(const DgJobDev& job) {
         const uint4 q0 = __ldcg(qs), q1 = __ldcg(qs + 1);
         const DgTriRec* R = job.trec + q0.x;
         EdgeSet e;
-        load_edges(R, e);
+        load_edges<true>(R, e);
         const float4 dd = __ldg(reinterpret_cast<const float4*>(R) + 4);
         const uint32_t seq = q0.y;
         const DgFrameDev& fr = job.frames[q0.z];
@@ -1230,7 +1230,7 @@ __device__ __forceinline__ void dev_resolve_tile(const DgJobDev& job, const DgFr
         const DgSmallRec* lean = LAZY && (rec & DG_LEAN) ? job.small + (rec & ~DG_LEAN) : nullptr;
         const float4* wp =
             EXT && (fr.flags & DG_FRAME_PERSPECTIVE) && job.trec_w && !lean ? job.trec_w + rec : nullptr;
-        uint32_t c = shade_from_record<EXT, LAZY>(job, fr, job.trec + rec, px, py, inv255, stex, d, errc, wp, lean);
+        uint32_t c = shade_from_record<EXT, LAZY, true>(job, fr, job.trec + rec, px, py, inv255, stex, d, errc, wp, lean);
         if (errc != DG_OK) {
             c = AZUL_BB;
             errors |= 1u << errc;

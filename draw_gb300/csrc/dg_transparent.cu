@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(256, DG_TRASTER_BLOCKS_PER_SM) k_traster(const
             y = bxy[lane] >> 16;
             const DgTriRec* R = job.ttrec + rec;
             EdgeSet e;
-            load_edges(R, e);
+            load_edges<false>(R, e);
             float al, be, ga;
             if (covered(e, (float)x, (float)y, al, be, ga)) {
                 fr = job.frames + __ldcg(&job.tbox[rec].w);
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(256, DG_TRASTER_BLOCKS_PER_SM) k_traster(const
             float d;
             int errc;
             const float4* wp = EXT && (fr->flags & DG_FRAME_PERSPECTIVE) && job.ttrec_w ? job.ttrec_w + rec : nullptr;
-            const uint32_t c = shade_from_record<EXT, false>(job, *fr, job.ttrec + rec, x, y, inv255, stex, d, errc, wp, nullptr);
+            const uint32_t c = shade_from_record<EXT, false, false>(job, *fr, job.ttrec + rec, x, y, inv255, stex, d, errc, wp, nullptr);
             if (errc != DG_OK) atomicOr(job.err, 1u << errc);
             link_fragment(job.fnode, job.fhead + pix, slot, key, c, __ldcg(job.talpha + rec));
         }
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(256, DG_TRASTER_BLOCKS_PER_SM) k_traster(const
             wi += nwarps;
             if (item.y >= item.z) continue;
             box = __ldcg(job.tbox + item.x);
-            load_edges(job.ttrec + item.x, e);
+            load_edges<false>(job.ttrec + item.x, e);
             fast = (e.tie & DG_EDGE_FAST) != 0u;
             // this lane's pixel of the box, stepped by DG_UNIT_PX pixels per unit (as in the opaque raster)
             k = item.y * DG_UNIT_PX + lane;
