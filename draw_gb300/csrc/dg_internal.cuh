@@ -460,7 +460,12 @@ bool dg_timeline_copy(unsigned long long* out, cudaStream_t s, cudaError_t* err)
 // dg_launch_job: part 0 after the opaque setup (painter's sort, gather,
 // transparent setup), part 1 after the opaque raster (fragment emission and
 // sort), part 2 after the opaque resolve (the ordered blend).
-cudaError_t dg_launch_transparent(int part, const DgJobDev& job, const DgTransparentPlan& plan, cudaStream_t s);
+// sorted (part 0): the painter's sort was launched by dg_launch_tsort_first.
+cudaError_t dg_launch_transparent(int part, const DgJobDev& job, const DgTransparentPlan& plan, cudaStream_t s,
+                                  bool sorted = false);
+// The painter's sort as the first kernel of a job with k_front (plan.tsort_meshes > 0).
+template <class IN>
+cudaError_t dg_launch_tsort_first(const IN& in, const DgTransparentPlan& plan, cudaStream_t s);
 
 // One batch of 2D overlay triangles (Canvas::draw_triangle, canvas.rs:435-575)
 // drawn into one canvas in order. The host clips every triangle's bounding box

@@ -671,6 +671,8 @@ __global__ void __launch_bounds__(DG_FRONT_THREADS) k_front(const __grid_constan
     auto frame = [&](uint32_t i) -> const DgFrameDev& { return in.frames[IN::kFrames == 1u ? 0u : i]; };
     dev_setup<true>(job, in.nsegs, seg, frame);
     dev_vertex<false>(job, in.nsegs, seg, frame);
+    // After k_tsort_first, the kernels behind this one need both complete (no wait otherwise).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Row of pixel k (row-major) of a box whose width's reciprocal is rw:
@@ -1379,6 +1381,7 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     };
     const bool front =
         cfg.front && (cfg.inl || cfg.inl_batch || cfg.inl_large) && job.total_vtx && job.total_tri;
+    const bool sort_first = front && job.ntt && cfg.tplan.tsort_meshes;
     if (job.total_vtx && !front) {
         NvtxRange r("k_vertex");
         const unsigned vb = cfg.vertex_blocks < 1u ? 1u : cfg.vertex_blocks;
@@ -1395,8 +1398,16 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     if (front) {
         NvtxRange r("k_front");
         const uint32_t blocks = (job.total_tri + DG_FRONT_THREADS - 1u) / DG_FRONT_THREADS;
-        with_inline([&](const auto& in) { k_front<<<blocks, DG_FRONT_THREADS, 0, s>>>(job, in); });
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        with_inline([&](const auto& in) {
+            if (sort_first) {
+                if ((e = dg_launch_tsort_first(in, cfg.tplan, s)) == cudaSuccess)
+                    e = launch_dependent(k_front<std::decay_t<decltype(in)>>, blocks, DG_FRONT_THREADS, job, s, in);
+            } else {
+                k_front<<<blocks, DG_FRONT_THREADS, 0, s>>>(job, in);
+                e = cudaGetLastError();
+            }
+        });
+        if (e != cudaSuccess) return e;
     } else if (job.total_tri) {
         NvtxRange r("k_setup_raster");
         if (job.lazy) {
@@ -1409,7 +1420,7 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     if ((e = mark(3)) != cudaSuccess) return e;
     // transparent pass, part 0: painter's sort and setup (its vertices join the
     // lighting prologue of the queue pass)
-    if ((e = dg_launch_transparent(0, job, cfg.tplan, s)) != cudaSuccess) return e;
+    if ((e = dg_launch_transparent(0, job, cfg.tplan, s, sort_first)) != cudaSuccess) return e;
     if (job.total_tri || job.ntt) {
         NvtxRange r("k_queue_raster");
         // Blocks beyond a job's possible work only cost their launch: at most a warp per

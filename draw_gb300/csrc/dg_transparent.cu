@@ -191,12 +191,12 @@ __device__ __forceinline__ uint32_t painter_key(const DgSegDev& sg, const DgFram
 // wide exchange steps; those within 64 keys stay inside a warp. For meshes of at
 // most DG_TSORT_MAX triangles it replaces k_tkeys, six or more radix passes of
 // three kernels and k_tgather (24 meshes of 800 triangles: 210 us).
-__global__ void __launch_bounds__(1024) k_tsort(const DgJobDev job) {
+template <class SEG, class FRM>
+__device__ __forceinline__ void dev_tsort(uint32_t nsegs, SEG seg, FRM frame) {
     extern __shared__ uint64_t s_key[];
-    wait_previous_kernel();
     const uint32_t mesh = blockIdx.x;
-    const DgSegDev& sg = job.segs[last_le(job.nsegs, mesh, [&](uint32_t i) { return job.segs[i].tmesh_base; })];
-    const DgFrameDev& fr = job.frames[sg.frame];
+    const DgSegDev& sg = seg(last_le(nsegs, mesh, [&](uint32_t i) { return seg(i).tmesh_base; }));
+    const DgFrameDev& fr = frame(sg.frame);
     const uint32_t first = __ldg(sg.tmesh_off + (mesh - sg.tmesh_base));
     const uint32_t n = __ldg(sg.tmesh_off + (mesh - sg.tmesh_base) + 1u) - first;
     uint32_t n2 = 64u;  // keys sorted: a power of two, at least one warp's
@@ -225,6 +225,23 @@ __global__ void __launch_bounds__(1024) k_tsort(const DgJobDev job) {
 #pragma unroll
         for (int k = 0; k < 3; k++) sg.tdst[k][first + i] = __ldg(sg.tsrc[k] + src);
     }
+}
+
+__global__ void __launch_bounds__(1024) k_tsort(const __grid_constant__ DgJobDev job) {
+    wait_previous_kernel();
+    dev_tsort(job.nsegs, [&](uint32_t i) -> const DgSegDev& { return job.segs[i]; },
+              [&](uint32_t i) -> const DgFrameDev& { return job.frames[i]; });
+}
+// The same as the first kernel of a job with k_front, on the descriptors that
+// travel with the job: neither reads what the other writes, so k_front starts
+// under it (and waits for it at its end, so that the kernels after k_front find
+// both complete). Measured on a 1280x720 frame with 24 transparent meshes of 812
+// triangles: the frame 168.7 -> 160.5 us.
+template <class IN>
+__global__ void __launch_bounds__(1024) k_tsort_first(const __grid_constant__ IN in) {
+    allow_next_kernel();  // the first kernel of a job waits on nothing (a stream-ordered launch)
+    dev_tsort(in.nsegs, [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; },
+              [&](uint32_t i) -> const DgFrameDev& { return in.frames[IN::kFrames == 1u ? 0u : i]; });
 }
 
 // Keys of the radix sort: the painter's key behind the job-wide index of the
@@ -846,15 +863,31 @@ cudaError_t dg_launch_overlay(const DgOverlayJob& job, unsigned blocks, cudaStre
     return launch_dependent(k_o_fold, g * 4u, 256, job, s);
 }
 
-cudaError_t dg_launch_transparent(int part, const DgJobDev& job, const DgTransparentPlan& plan, cudaStream_t s) {
+namespace {
+unsigned tsort_threads(const DgTransparentPlan& plan) {
+    return plan.tsort_pow2 / 2u < 1024u ? plan.tsort_pow2 / 2u : 1024u;
+}
+}  // namespace
+
+template <class IN>
+cudaError_t dg_launch_tsort_first(const IN& in, const DgTransparentPlan& plan, cudaStream_t s) {
+    k_tsort_first<<<plan.tsort_meshes, tsort_threads(plan), plan.tsort_pow2 * sizeof(uint64_t), s>>>(in);
+    return cudaGetLastError();
+}
+template cudaError_t dg_launch_tsort_first(const DgInlineDesc&, const DgTransparentPlan&, cudaStream_t);
+template cudaError_t dg_launch_tsort_first(const DgInlineBatch&, const DgTransparentPlan&, cudaStream_t);
+template cudaError_t dg_launch_tsort_first(const DgInlineLarge&, const DgTransparentPlan&, cudaStream_t);
+
+cudaError_t dg_launch_transparent(int part, const DgJobDev& job, const DgTransparentPlan& plan, cudaStream_t s,
+                                  bool sorted) {
     if (job.ntt == 0u) return cudaSuccess;
     const unsigned g = plan.blocks < 1u ? 1u : plan.blocks;
     cudaError_t e = cudaSuccess;
     if (part == 0) {
-        if (plan.tsort_meshes) {
-            const unsigned threads = plan.tsort_pow2 / 2u < 1024u ? plan.tsort_pow2 / 2u : 1024u;
-            if ((e = launch_dependent_smem(k_tsort, plan.tsort_meshes, threads, plan.tsort_pow2 * sizeof(uint64_t), job,
-                                           s)) != cudaSuccess)
+        if (sorted) {  // by dg_launch_tsort_first
+        } else if (plan.tsort_meshes) {
+            if ((e = launch_dependent_smem(k_tsort, plan.tsort_meshes, tsort_threads(plan),
+                                           plan.tsort_pow2 * sizeof(uint64_t), job, s)) != cudaSuccess)
                 return e;
         } else {
             if ((e = launch_dependent(k_tkeys, grid_for(job.ntt, g), 256, job, s)) != cudaSuccess) return e;
