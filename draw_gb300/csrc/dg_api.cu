@@ -868,8 +868,8 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
         DG_CUDA(cudaMallocHost(&S.h_stage[k], stage_cap));
         S.h_stage_cap[k] = stage_cap;
     }
-    // A small job's descriptors go to the device as a kernel parameter (k_vertex
-    // writes them to the staging buffer); larger ones are copied.
+    // A small job's descriptors go to the device as a parameter of its first
+    // kernel (which writes them to the staging buffer); larger ones are copied.
     DgInlineDesc inl;
     DgInlineBatch inl_batch;
     DgInlineLarge inl_large;

@@ -12,7 +12,8 @@
 //   render scratch: vrec float4[V_total] (snapped centre x,y, eye distance,
 //                   plane-sign masks), vmask u16[V_total] (the masks alone, for
 //                   the cull's gathers), vshade float4[V_total*L*2] (light, halfway),
-//                   raster-queue records + their work-unit bases, counters
+//                   triangle records, raster-queue records and their work items,
+//                   the small-triangle list, two sets of counters
 #pragma once
 
 #include <cstddef>
@@ -54,7 +55,7 @@ __device__ __forceinline__ bool dg_check_range(bool ok, uint32_t* err) {
 
 // Triangles whose clipped bounding box has at most DgFrameDev.small_max_px
 // pixels go to the small-triangle list, whose entries the queue pass rasterizes
-// 32 at a time per warp, their boxes' pixels numbered together; larger ones go to
+// 32 at a time per warp (raster_small_chunk); larger ones go to
 // the raster queue: their bounding box is cut into work items (DgItemGrid) of
 // about 2^DgJobDev.item_log2 pixels (128 * item_units, default DG_ITEM_UNITS),
 // which the queue pass spreads over all warps. Unless the tuning fixes it, a

@@ -5,15 +5,17 @@
 //                   screen centre, plane-sign masks (scene/mod.rs:917-926,
 //                   :1047-1058, canvas.rs:585-587)
 //   k_cull          per input triangle: lateral and near reject from the sign
-//                   masks, back-face cull; survivors are compacted
+//                   masks, back-face cull, triangles without area; survivors are
+//                   compacted
+//   k_setup_lean    (frames of micro triangles) list entries of the small
+//                   unclipped survivors, which get no record
 //   k_setup_raster  per survivor: near/far clipping, triangle records, bounding
-//                   box, edge functions; tiny triangles are rasterized by their
-//                   warp (pixels of all 32 lanes' boxes flattened with a warp
-//                   prefix scan), the others are queued (scene/mod.rs:933-1063,
-//                   canvas.rs:585-681)
-//   k_queue_raster  light/halfway vectors of the marked vertices, then the
-//                   queued triangles' bounding-box pixels in 32-pixel units
-//                   spread evenly over all warps
+//                   box, edge functions; small triangles go to a list, the others
+//                   to the queue (scene/mod.rs:933-1063, canvas.rs:585-681)
+//   (k_front        all of these in one kernel, for small jobs)
+//   k_queue_raster  light/halfway vectors of the marked vertices, then the small
+//                   triangles 32 per warp, then the queued ones by parts of their
+//                   boxes, whose covered row spans are finished 32 pixels at a time
 //   k_resolve       per 32 x tile_rows tile: a tile that no triangle box reached
 //                   (its 32x32 cell lacks the frame's epoch) gets the clear
 //                   values without reading its keys; otherwise empty pixels
@@ -42,7 +44,7 @@ namespace {
 // block-uniform loops) wrapped by its kernel; the five kernels run as a chain
 // with programmatic dependent launch.
 // seg(i) and frame(i) give the job's descriptors (from global memory, or from
-// k_vertex's parameter for a small job).
+// the first kernel's parameter for a small job).
 #if DG_TIMELINE
 // [kernel][first start, first wait passed, last wait passed, last end]
 __device__ unsigned long long g_timeline[DG_NKERNELS][4] = {

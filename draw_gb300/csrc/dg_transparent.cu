@@ -20,10 +20,11 @@
 // fragments that come from an object at or after j*'s and whose depth is < d*
 // (d* = the clear depth and every object qualifies when no opaque fragment
 // covers the pixel). The pass:
-//   part 0 (after the opaque setup): per-mesh painter's sort keys, a stable LSD
-//          radix sort, the permutation of the triangle arrays into the new
-//          persistent order, and the transparent setup (clipping, triangle
-//          records, bounding boxes, vertices marked for lighting);
+//   part 0 (after the opaque setup; the sort beside it in a job with k_front):
+//          the painter's sort of each mesh (one block per mesh in shared memory,
+//          or keys, a stable LSD radix sort and the permutation for larger ones)
+//          into the new persistent order, and the transparent setup (clipping,
+//          triangle records, bounding boxes, vertices marked for lighting);
 //   part 1 (after the opaque raster, while the visibility keys still hold j*):
 //          the work items of the outputs' bounding boxes are rasterized with the
 //          exact coverage test, and every qualifying fragment is shaded and
