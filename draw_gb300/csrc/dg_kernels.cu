@@ -1031,7 +1031,13 @@ __global__ void __launch_bounds__(256, 4) k_queue_raster(const DgJobDev job) {
     DG_TL_BLOCK(3);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     DG_TL_WAITED(3);
-    if (job.split_below) count_reached_cells(job);
+    if (job.split_below) {
+        count_reached_cells(job);
+        // A block's launch signal is the first one that any of its threads gives, so
+        // all of them must have counted: without the barrier k_resolve_split's blocks
+        // could read different partial counts and disagree on strips.
+        __syncthreads();
+    }
     allow_next_kernel();
     dev_queue(job);
 }
