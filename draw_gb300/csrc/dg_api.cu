@@ -374,9 +374,9 @@ dg_status slot_init(dg_ctx* c, JobSlot& s, cudaStream_t stream) {
     s.stream = stream;
     for (int i = 0; i < JobSlot::kStage; i++) DG_CUDA(cudaEventCreateWithFlags(&s.stage_ev[i], cudaEventDisableTiming));
     for (int i = 0; i <= DG_NKERNELS; i++) DG_CUDA(cudaEventCreate(&s.ev[i]));
-    dg_status e = dalloc(&s.d_counters, 2 * DG_NCOUNTERS);
+    dg_status e = dalloc(&s.d_counters, 3 * DG_NCOUNTERS);
     if (e) return e;
-    DG_CUDA(cudaMemsetAsync(s.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), stream));
+    DG_CUDA(cudaMemsetAsync(s.d_counters, 0, 3 * DG_NCOUNTERS * sizeof(unsigned long long), stream));
     e = dalloc(&s.d_err, 1);
     if (e) return e;
     DG_CUDA(cudaMemset(s.d_err, 0, 4));
@@ -832,7 +832,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
 dg_status enqueue_job(JobBuild& B, JobSlot& S, void* d_stage, cudaStream_t stream, bool timing) {
     B.job.frames = (const DgFrameDev*)d_stage;
     B.job.segs = (const DgSegDev*)((uint8_t*)d_stage + B.fbytes);
-    if (!B.job.total_vtx)  // otherwise the first kernel does
+    if (!B.job.total_vtx && B.job.cnt_next)  // otherwise the first kernel does
         DG_CUDA(cudaMemsetAsync(B.job.cnt_next, 0, DG_NCOUNTERS * sizeof(unsigned long long), stream));
     DG_CUDA(dg_launch_job(B.job, B.cfg, stream, timing ? S.ev : nullptr));
     return DG_OK;
@@ -848,11 +848,24 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
     B.inline_ok = true;
     dg_status e = build_job(c, S, scenes, targets, n, B);
     if (e) return e;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    DG_CUDA(cudaStreamIsCapturing(S.stream, &cs));
+    const bool captured = cs != cudaStreamCaptureStatusNone;
+    if (captured) {
+        // The caller captures this job into a graph of its own: a replay follows
+        // whatever ran last, itself for instance, so the job zeroes its counters
+        // (a set that other jobs do not use) and leaves the next job's alone.
+        B.job.cnt = S.d_counters + JobSlot::kCapturedSet * DG_NCOUNTERS;
+        B.job.cnt_next = nullptr;
+    }
     // job descriptor upload through a pinned staging slot
     const size_t need = B.fbytes + B.sbytes;
     const int k = S.stage;
     S.stage = (S.stage + 1) % JobSlot::kStage;
-    DG_CUDA(cudaEventSynchronize(S.stage_ev[k]));
+    // (an event recorded in a capture cannot be waited for later, and descriptors
+    // that travel with the first kernel use no pinned buffer)
+    const bool stage_event = !(captured && B.inline_desc);
+    if (stage_event) DG_CUDA(cudaEventSynchronize(S.stage_ev[k]));
     const size_t stage_cap = std::max<size_t>(need * 2, 64 * 1024);
     if (S.stage_cap[k] < need) {
         dfree(S.d_stage[k]);
@@ -894,21 +907,26 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
         std::memcpy((uint8_t*)S.h_stage[k] + B.fbytes, B.segs.data(), B.sbytes);
         DG_CUDA(cudaMemcpyAsync(S.d_stage[k], S.h_stage[k], need, cudaMemcpyHostToDevice, S.stream));
     }
-    DG_CUDA(cudaEventRecord(S.stage_ev[k], S.stream));
+    if (stage_event) DG_CUDA(cudaEventRecord(S.stage_ev[k], S.stream));
     S.last_vtx = B.total_vtx;
     S.last_tri = B.total_tri;
     S.last_h2d = need;
     S.last_launches = B.launches;
     S.last_tile_rows = B.job.tile_rows;
     S.last_small_max_px = B.frames.empty() ? 0 : B.frames[0].small_max_px;
+    if (captured) DG_CUDA(cudaMemsetAsync(B.job.cnt, 0, DG_NCOUNTERS * sizeof(unsigned long long), S.stream));
     e = enqueue_job(B, S, S.d_stage[k], S.stream, S.timing);
     if (e) {  // part of the job may have run: start over with zero counters
-        cudaMemsetAsync(S.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), S.stream);
+        if (!captured) cudaMemsetAsync(S.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), S.stream);
         cudaGetLastError();
         return e;
     }
-    S.last_set = S.cnt_set;
-    S.cnt_set ^= 1;
+    if (captured) {
+        S.last_set = JobSlot::kCapturedSet;
+    } else {
+        S.last_set = S.cnt_set;
+        S.cnt_set ^= 1;
+    }
     advance_transparent(c, B);
     if (S.timing) S.ev_valid = true;
     return DG_OK;

@@ -179,7 +179,9 @@ struct JobSlot {
     uint32_t item_units = DG_ITEM_UNITS;
     uint32_t record_limit = 0;
     // Two sets of job counters (DG_CNT_*, DG_NCOUNTERS words each): jobs alternate,
-    // and a job's first kernel zeroes the other set for the job after it.
+    // and a job's first kernel zeroes the other set for the job after it. A third
+    // one is for jobs that the caller captures into a graph, which zero it themselves.
+    static const int kCapturedSet = 2;
     unsigned long long* d_counters = nullptr;
     int cnt_set = 0;   // the next job's set
     int last_set = 0;  // the last job's set
