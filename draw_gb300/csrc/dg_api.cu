@@ -1631,6 +1631,11 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
         nitems += (units + step - 1) / step;
     }
     if (total >= 0x7FFFFFFFull) return DG_E_LIMIT;
+    // Not into a graph of the caller's: a replay would read the pinned buffer of this
+    // call, which later calls fill again.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    DG_CUDA(cudaStreamIsCapturing(c->main.stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) return DG_E_CUDA;
     JobSlot& S = c->main;
     const unsigned blocks = (unsigned)c->nsm * DG_OVERLAY_BLOCKS_PER_SM;
     const size_t o_verts = 16, o_box = o_verts + 96ull * n, o_items = o_box + 16ull * n, bytes = o_items + 8 * nitems;

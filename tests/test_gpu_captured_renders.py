@@ -92,3 +92,36 @@ def test_replays(name, oracle_lib):
     finally:
         ctx.set_stream(None)
         ctx.close()
+
+
+def test_overlay_is_refused_in_a_capture(oracle_lib):
+    """A graph would read the call's staging buffer at every replay: refused, and the
+    context works on."""
+    import torch
+    from draw_gb300 import renderer
+
+    ctx = renderer.Context(0)
+    try:
+        stream = torch.cuda.Stream()
+        ctx.set_stream(stream.cuda_stream)
+        canvas = renderer.Canvas(64, 48, ctx)
+        canvas.init_depth(1.0e9)
+        verts = np.zeros((1, 3, 8), np.float32)
+        verts[0, :, :2] = [[2, 2], [60, 2], [2, 40]]
+        verts[..., 4:7], verts[..., 7] = 200.0, 0.5
+        atlas = renderer.TextureMap(np.full(8 * 8 * 4, 255, np.uint8), 8, 8, 4, ctx)
+        canvas.draw_triangles(verts, atlas)  # allocates the scratch
+        before = canvas.read()[0].copy()
+        graph = torch.cuda.CUDAGraph()
+        with pytest.raises(renderer.DrawError) as err:
+            with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+                torch.zeros(1, device="cuda")  # the graph is not empty
+                canvas.draw_triangles(verts, atlas)
+        assert err.value.status == 6  # DG_E_CUDA
+        assert np.array_equal(before, canvas.read()[0])
+        canvas.draw_triangles(verts, atlas)
+        assert not np.array_equal(before, canvas.read()[0])
+        torch.cuda.synchronize()
+    finally:
+        ctx.set_stream(None)
+        ctx.close()
