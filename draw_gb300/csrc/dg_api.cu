@@ -11,6 +11,7 @@
 #include <cstring>
 #include <memory>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "dg_host.h"
@@ -467,6 +468,18 @@ size_t queue_records(uint64_t total_tri) {
 // resolve pass shades the pixels of triangles without a record the long way).
 size_t trec_records(uint64_t total_tri) { return (size_t)std::min<uint64_t>(dg_trec_cap(total_tri), 0xFFFFFFF0ull); }
 
+// Zeroes what every job of a slot expects to be zero, after one that did not run to
+// its end. On a capturing stream nothing runs now, so the slot stays dirty.
+static dg_status slot_reset(JobSlot& S) {
+    DG_CUDA(cudaMemsetAsync(S.d_counters, 0, 3 * DG_NCOUNTERS * sizeof(unsigned long long), S.stream));
+    if (S.d_fhead) DG_CUDA(cudaMemsetAsync(S.d_fhead, 0, S.fhead_cap * sizeof(uint32_t), S.stream));
+    if (S.d_vmark) DG_CUDA(cudaMemsetAsync(S.d_vmark, 0, S.vmark_cap * sizeof(uint8_t), S.stream));
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    DG_CUDA(cudaStreamIsCapturing(S.stream, &cs));
+    S.dirty = cs != cudaStreamCaptureStatusNone;
+    return DG_OK;
+}
+
 uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L, uint64_t P) {
     auto cap_after = [](size_t cap, const void* p, size_t need) -> size_t {
         return (cap >= need && p) ? cap : std::max(need, cap * 3 / 2);
@@ -490,6 +503,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
                     JobBuild& B) {
     dg_status e = set_device(c);
     if (e) return e;
+    if (S.dirty && (e = slot_reset(S))) return e;
     std::vector<DgFrameDev>& frames = B.frames;
     std::vector<DgSegDev>& segs = B.segs;
     frames.assign(n, DgFrameDev{});
@@ -693,7 +707,9 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         if (S.fhead_cap < total_px) {
             e = grow(S, &S.d_fhead, &S.fhead_cap, total_px);
             if (e) return e;
+            S.dirty = true;  // until the memset is on its way
             DG_CUDA(cudaMemsetAsync(S.d_fhead, 0, S.fhead_cap * sizeof(uint32_t), S.stream));
+            S.dirty = false;
         }
         const uint64_t tiles = (ntt + DG_SORT_TILE - 1) / DG_SORT_TILE;
         e = grow(S, &S.d_hist, &S.hist_cap, 256 * tiles);
@@ -717,7 +733,9 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     if (S.vmark_cap < want_mark) {
         e = grow(S, &S.d_vmark, &S.vmark_cap, want_mark);
         if (e) return e;
+        S.dirty = true;
         DG_CUDA(cudaMemsetAsync(S.d_vmark, 0, S.vmark_cap * sizeof(uint8_t), S.stream));
+        S.dirty = false;
     }
     const size_t want_queue = queue_records(total_tri);
     if (S.queue_cap < want_queue) {
@@ -915,10 +933,20 @@ dg_status launch_frames(dg_ctx* c, JobSlot& S, Scene* const* scenes, const Frame
     S.last_tile_rows = B.job.tile_rows;
     S.last_small_max_px = B.frames.empty() ? 0 : B.frames[0].small_max_px;
     if (captured) DG_CUDA(cudaMemsetAsync(B.job.cnt, 0, DG_NCOUNTERS * sizeof(unsigned long long), S.stream));
+    B.cfg.fail_before = S.fail_before;
+    S.fail_before = 0;
     e = enqueue_job(B, S, S.d_stage[k], S.stream, S.timing);
-    if (e) {  // part of the job may have run: start over with zero counters
-        if (!captured) cudaMemsetAsync(S.d_counters, 0, 2 * DG_NCOUNTERS * sizeof(unsigned long long), S.stream);
+    if (e) {
+        // Part of the job may have run. Its kernels leave to later ones to clear the
+        // visibility keys, fragment list heads, vertex marks and counters: a list head
+        // left behind would join the next job's nodes to a stale one, or to themselves.
         cudaGetLastError();
+        if (!captured) {
+            S.dirty = true;
+            for (uint32_t i = 0; i < n; i++)
+                cudaMemsetAsync(targets[i].vis, 0xFF, targets[i].w * targets[i].h * sizeof(uint64_t), S.stream);
+            cudaGetLastError();
+        }
         return e;
     }
     if (captured) {
@@ -1049,6 +1077,13 @@ dg_status dg_ctx_set_timing(dg_ctx* c, int32_t enable) {
     if (!c) return DG_E_INVALID;
     c->main.timing = enable != 0;
     c->main.ev_valid = false;
+    return DG_OK;
+}
+
+dg_status dg_ctx_inject_launch_failure(dg_ctx* c, int32_t before) {
+    if (!c || before < 0 || before > 9) return DG_E_INVALID;
+    c->main.fail_before = before < 9 ? before : 0;
+    c->overlay.fail_launch = before == 9;
     return DG_OK;
 }
 
@@ -1644,7 +1679,11 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
         return e;
     if (O.head_cap < cv->w * cv->h) {
         if ((e = grow(S, &O.d_head, &O.head_cap, cv->w * cv->h))) return e;
+        O.dirty = true;
+    }
+    if (O.dirty) {  // new heads, or some that a batch without its blend left behind
         DG_CUDA(cudaMemsetAsync(O.d_head, 0, O.head_cap * sizeof(uint32_t), S.stream));
+        O.dirty = false;
     }
     const int k = O.stage;
     O.stage = (O.stage + 1) % OverlaySlot::kStage;
@@ -1695,7 +1734,9 @@ dg_status dg_canvas_draw_triangles_2d(dg_ctx* c, int32_t canvas, const float* ve
     j.head = O.d_head;
     j.err = S.d_err;
     for (uint32_t b = n - 1; b; b >>= 1) j.key_bits++;
-    DG_CUDA(dg_launch_overlay(j, blocks, S.stream));
+    O.dirty = true;  // until the blend, which clears the heads, is on its way
+    DG_CUDA(dg_launch_overlay(j, blocks, S.stream, std::exchange(O.fail_launch, false)));
+    O.dirty = false;
     return DG_OK;
 }
 

@@ -255,6 +255,7 @@ dg_status dg_batch_render(dg_batch* b) {
     if (ge != cudaSuccess) {  // the next replay captures again, with zero counters
         cudaGetLastError();
         drop_graphs(b);
+        b->slot.dirty = true;
         return ge == cudaErrorMemoryAllocation ? DG_E_OOM : DG_E_CUDA;
     }
     DG_CUDA(cudaEventRecord(b->done[k], c->main.stream));

@@ -193,6 +193,10 @@ struct JobSlot {
     size_t h_stage_cap[kStage] = {};  // bytes of h_stage (inline descriptors need none)
     cudaEvent_t stage_ev[kStage] = {};
     int stage = 0;
+    // Set when a job may have left state behind that jobs expect to be zero (counters,
+    // fhead, vmark): build_job clears it all before the next job.
+    bool dirty = false;
+    int32_t fail_before = 0;  // dg_ctx_inject_launch_failure, for the next job
     bool timing = false;
     cudaEvent_t ev[DG_NKERNELS + 1] = {};
     bool ev_valid = false;
@@ -222,6 +226,8 @@ struct OverlaySlot {
     size_t node_cap = 0;
     uint32_t* d_head = nullptr;  // zeroed at allocation; the fold clears what the raster sets
     size_t head_cap = 0;
+    bool dirty = false;        // a batch may have left heads behind: cleared before the next one
+    bool fail_launch = false;  // dg_ctx_inject_launch_failure, for the next batch
     uint32_t* d_rgba = nullptr;  // staging of dg_canvas_read_rgba
     size_t rgba_cap = 0;
 };

@@ -416,6 +416,7 @@ struct DgLaunchCfg {
     const DgInlineBatch* inl_batch;
     const DgInlineLarge* inl_large;
     bool front;  // with one of them: k_front in place of the vertex, cull and setup passes
+    int32_t fail_before;  // not 0: dg_ctx_inject_launch_failure
     DgTransparentPlan tplan;
 };
 // k_vertex's grid cap: its resident blocks (launch bounds 256 x 8), one wave
@@ -496,8 +497,8 @@ constexpr uint32_t dg_overlay_units(uint64_t npx) {
     return per < 4u ? 4u : (uint32_t)per;
 }
 #define DG_OVERLAY_BLOCKS_PER_SM 4u
-// blocks: the raster's grid (node_cap is sized for it).
-cudaError_t dg_launch_overlay(const DgOverlayJob& job, unsigned blocks, cudaStream_t s);
+// blocks: the raster's grid (node_cap is sized for it). fail: dg_ctx_inject_launch_failure.
+cudaError_t dg_launch_overlay(const DgOverlayJob& job, unsigned blocks, cudaStream_t s, bool fail = false);
 // Scratch rows and records sized for a job of T triangles (shared sizing rule).
 constexpr uint64_t dg_trec_cap(uint64_t T) { return T + T / 8u + 4096u; }
 constexpr uint64_t dg_items_cap(uint64_t queue_cap) { return 2u * queue_cap + 65536u; }

@@ -1375,6 +1375,8 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     NvtxRange job_range("draw_gb300 render job");
     cudaError_t e;
     auto mark = [&](int i) { return ev ? cudaEventRecord(ev[i], s) : cudaSuccess; };
+    // dg_ctx_inject_launch_failure: the job ends before launch k
+    auto refused = [&](int32_t k) { return cfg.fail_before == k ? cudaErrorMemoryAllocation : cudaSuccess; };
     if ((e = mark(0)) != cudaSuccess) return e;
     DgInlineDesc none;
     none.nsegs = 0;
@@ -1390,19 +1392,20 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
     const bool front =
         cfg.front && (cfg.inl || cfg.inl_batch || cfg.inl_large) && job.total_vtx && job.total_tri;
     const bool sort_first = front && job.ntt && cfg.tplan.tsort_meshes;
+    if ((e = refused(1)) != cudaSuccess) return e;
     if (job.total_vtx && !front) {
         NvtxRange r("k_vertex");
         const unsigned vb = cfg.vertex_blocks < 1u ? 1u : cfg.vertex_blocks;
         with_inline([&](const auto& in) { k_vertex<<<grid_for(job.total_vtx, vb), 256, 0, s>>>(job, in); });
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if ((e = mark(1)) != cudaSuccess) return e;
+    if ((e = mark(1)) != cudaSuccess || (e = refused(2)) != cudaSuccess) return e;
     if (job.total_tri && !front) {
         NvtxRange r("k_cull");
         const unsigned cb = cfg.cull_blocks < 1u ? 1u : cfg.cull_blocks;
         if ((e = launch_dependent(k_cull, grid_for(job.total_tri, cb), 256, job, s)) != cudaSuccess) return e;
     }
-    if ((e = mark(2)) != cudaSuccess) return e;
+    if ((e = mark(2)) != cudaSuccess || (e = refused(3)) != cudaSuccess) return e;
     if (front) {
         NvtxRange r("k_front");
         const uint32_t blocks = (job.total_tri + DG_FRONT_THREADS - 1u) / DG_FRONT_THREADS;
@@ -1425,10 +1428,11 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
         const unsigned sb = cfg.setup_blocks < 1u ? 1u : cfg.setup_blocks;
         if ((e = launch_dependent(k_setup_raster, grid_for(job.total_tri, sb), 256, job, s)) != cudaSuccess) return e;
     }
-    if ((e = mark(3)) != cudaSuccess) return e;
+    if ((e = mark(3)) != cudaSuccess || (e = refused(4)) != cudaSuccess) return e;
     // transparent pass, part 0: painter's sort and setup (its vertices join the
     // lighting prologue of the queue pass)
     if ((e = dg_launch_transparent(0, job, cfg.tplan, s, sort_first)) != cudaSuccess) return e;
+    if ((e = refused(5)) != cudaSuccess) return e;
     if (job.total_tri || job.ntt) {
         NvtxRange r("k_queue_raster");
         // Blocks beyond a job's possible work only cost their launch: at most a warp per
@@ -1438,9 +1442,10 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
         const unsigned qb = grid_for(qw * 32u, cfg.queue_blocks < 1u ? 1u : cfg.queue_blocks);
         if ((e = launch_dependent(k_queue_raster, qb, 256, job, s)) != cudaSuccess) return e;
     }
-    if ((e = mark(4)) != cudaSuccess) return e;
+    if ((e = mark(4)) != cudaSuccess || (e = refused(6)) != cudaSuccess) return e;
     // part 1: transparent fragments, read against the opaque winners' keys
     if ((e = dg_launch_transparent(1, job, cfg.tplan, s)) != cudaSuccess) return e;
+    if ((e = refused(7)) != cudaSuccess) return e;
     if (job.total_tiles) {
         NvtxRange r("k_resolve");
         using KR = void (*)(const DgJobDev);
@@ -1458,6 +1463,7 @@ cudaError_t dg_launch_job(const DgJobDev& job, const DgLaunchCfg& cfg, cudaStrea
         const unsigned grid = job.split_below ? 4u * job.total_tiles : job.total_tiles;
         if ((e = launch_dependent(kr, grid, 256, job, s)) != cudaSuccess) return e;
     }
+    if ((e = refused(8)) != cudaSuccess) return e;
     // part 2: the ordered blend over the opaque colours
     if ((e = dg_launch_transparent(2, job, cfg.tplan, s)) != cudaSuccess) return e;
     return mark(5);

@@ -219,7 +219,10 @@ dg_status launch_batch(dg_server* s, Slot* sl, std::vector<Request*>& batch, uin
     }
     dg_status e = launch_frames(s->ctx, sl->js, sc.data(), tg.data(), (uint32_t)batch.size());
     settle();
-    if (e) return e;
+    if (e) {  // what did launch must end before the caller gives the requests' buffers back
+        cudaStreamSynchronize(st);
+        return e;
+    }
     if (cudaMemcpyAsync(sl->h_err, sl->js.d_err, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return DG_E_CUDA;
     if (cudaMemsetAsync(sl->js.d_err, 0, 4, st) != cudaSuccess) return DG_E_CUDA;
     sl->batch = batch;

@@ -596,7 +596,10 @@ __device__ __forceinline__ uint32_t px_add(uint32_t p, uint32_t q) {
 
 // Puts a list of fragment nodes in ascending key order (a stable LSD radix sort
 // of the links, 4 bits per pass) and returns its head; for lists too long for
-// fold_list's registers.
+// fold_list's registers. Its walks end because every list does: heads are zero
+// before a job (JobSlot::dirty, OverlaySlot::dirty) and a job hands every node out
+// once. Counting the nodes against the number of keys in the loop doubled the
+// time of long lists (200 full-frame layers at 1920x1080: 22.4 -> 45.3 ms).
 __device__ __noinline__ uint32_t sort_list(uint4* node, uint32_t head, uint32_t key_bits) {
     for (uint32_t shift = 0; shift < key_bits; shift += 4u) {
         uint32_t hd[16], tl[16];
@@ -856,11 +859,12 @@ __global__ void __launch_bounds__(256) k_o_fold(const __grid_constant__ DgOverla
 
 }  // namespace
 
-cudaError_t dg_launch_overlay(const DgOverlayJob& job, unsigned blocks, cudaStream_t s) {
+cudaError_t dg_launch_overlay(const DgOverlayJob& job, unsigned blocks, cudaStream_t s, bool fail) {
     if (job.n == 0u) return cudaSuccess;
     const unsigned g = blocks < 1u ? 1u : blocks;
     const cudaError_t e = launch_dependent(k_o_raster, g, 256, job, s);
     if (e != cudaSuccess) return e;
+    if (fail) return cudaErrorMemoryAllocation;
     return launch_dependent(k_o_fold, g * 4u, 256, job, s);
 }
 

@@ -37,6 +37,7 @@ SIGNATURES = {
     "dg_ctx_stream": (_P, [_P]),
     "dg_ctx_set_timing": (_i32, [_P, _i32]),
     "dg_ctx_kernel_times": (_i32, [_P, _P, _i32]),
+    "dg_ctx_inject_launch_failure": (_i32, [_P, _i32]),
     "dg_timeline_read": (_i32, [_P, _P, _i32]),
     "dg_ctx_last_stats": (_i32, [_P, _P, _i32]),
     "dg_check_division": (_i32, [_P, _i32, _u64, _u64, _P, _P, _P]),
@@ -226,6 +227,10 @@ class Context:
         ms = (ctypes.c_float * len(KERNELS))()
         _chk(self.lib.dg_ctx_kernel_times(self.h, ms, len(KERNELS)), "kernel_times")
         return dict(zip(KERNELS, list(ms)))
+
+    def inject_launch_failure(self, before: int):
+        """dg_ctx_inject_launch_failure (test hook): the next job fails before this launch."""
+        _chk(self.lib.dg_ctx_inject_launch_failure(self.h, before), "inject_launch_failure")
 
     def timeline(self) -> dict:
         """dg_timeline_read (DRAW_TIMELINE builds): per kernel, microseconds after the

@@ -90,6 +90,14 @@ void* dg_ctx_stream(dg_ctx* ctx);
  * small frame's vertex, cull and setup passes are one kernel, timed as "setup_raster". */
 dg_status dg_ctx_set_timing(dg_ctx* ctx, int32_t enable);
 dg_status dg_ctx_kernel_times(dg_ctx* ctx, float* ms, int32_t n);
+/* Host-side fault injection for tests: the next dg_scene_render or dg_render_batch
+ * job of the context returns DG_E_OOM in place of one of its launches, as if the
+ * driver had refused it, with the launches before it already made. before: 1 vertex,
+ * 2 cull, 3 setup (or the one-kernel front), 4 transparent setup, 5 queue, 6 transparent
+ * fragments, 7 resolve, 8 transparent blend, a launch that the job does not have
+ * included; 9: the next dg_canvas_draw_triangles_2d, before its blend; 0: none. No GPU
+ * fault is involved. */
+dg_status dg_ctx_inject_launch_failure(dg_ctx* ctx, int32_t before);
 /* Kernel timeline of the render jobs since the last call, in builds made with
  * DRAW_TIMELINE (draw_gb300/_build.py build(timeline=True)); other builds
  * return DG_E_INVALID. out[4k .. 4k+3] for kernel k in the order of
