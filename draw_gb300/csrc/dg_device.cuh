@@ -519,13 +519,13 @@ __device__ __forceinline__ void light_halfway(const DgFrameDev& fr, V3 p, V3 eye
     h = vnormalized(vadd(lt, eye_n));
 }
 
-// 32 bytes of global memory by one instruction (two float4s side by side, 32-byte
+// 32 bytes of global memory by one load (two float4s side by side, 32-byte
 // aligned): a 16-byte access of strided lanes moves half a sector at a time.
-// Measured on 32 uneven frames (222,000 records): setup pass 38.9 -> 32.8 us with
-// 32-byte record stores, resolve 63.5 -> 61.4 with 32-byte loads. Only in code
-// inlined into the kernels: in the out-of-line clip functions the 32-byte store
-// left wrong records in jobs with many clipped triangles (the 16-byte stores of
-// the same values do not), so those keep 16-byte stores.
+// Measured on 32 uneven frames (222,000 records): resolve 63.5 -> 61.4 us. Stores
+// are of 16 bytes: in the out-of-line clip functions a 32-byte store of the same
+// values left wrong records, in inline assembly and as the compiler's own store of
+// a 32-byte vector type alike, for a reason that the source does not show. As the
+// setup kernels call these functions, none of their code uses it.
 __device__ __forceinline__ void ldg8(const float4* p, float4& a, float4& b) {
     asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -540,30 +540,16 @@ __device__ __forceinline__ void ldg_pair(const float4* p, float4& a, float4& b) 
         b = __ldg(p + 1);
     }
 }
-__device__ __forceinline__ void stg8(float4* p, float4 a, float4 b) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(__cvta_generic_to_global(p)),
-                 "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-                 : "memory");
-}
-__device__ __forceinline__ float4 as_float4(uint4 v) {
-    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
-}
 __device__ __forceinline__ uint4 as_uint4(float4 v) {
     return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
 }
 
 // Writes row `row` of the light/halfway table: per light l, float4s 2l and 2l+1
 // hold (lt.x, lt.y, lt.z, h.x) and (h.y, h.z, 0, 0).
-template <bool WIDE>
 __device__ __forceinline__ void put_shade(const DgJobDev& job, uint32_t row, uint32_t l, V3 lt, V3 h) {
     float4* dst = job.vshade + ((uint64_t)row * job.shade_stride + l) * 2;
-    const float4 w0 = make_float4(lt.x, lt.y, lt.z, h.x), w1 = make_float4(h.y, h.z, 0.0f, 0.0f);
-    if (WIDE) {
-        stg8(dst, w0, w1);
-    } else {
-        dst[0] = w0;
-        dst[1] = w1;
-    }
+    dst[0] = make_float4(lt.x, lt.y, lt.z, h.x);
+    dst[1] = make_float4(h.y, h.z, 0.0f, 0.0f);
 }
 
 // Light and halfway vectors of job vertex v for every light. Only vertices of
@@ -580,7 +566,7 @@ __device__ __forceinline__ void shade_vertex(const DgJobDev& job, uint32_t v) {
     for (uint32_t l = 0; l < fr.nlights; l++) {
         V3 lt, h;
         light_halfway(fr, p, eye, l, lt, h);
-        put_shade<true>(job, v, l, lt, h);
+        put_shade(job, v, l, lt, h);
     }
 }
 
@@ -604,26 +590,17 @@ __device__ __noinline__ void clip_shade_rows(const DgJobDev& job, const DgFrameD
         for (int k = 3; k < P.nv; k++)
             for (int c = 0; c < 6; c++) f[c][k] = fA(f[c][P.p[k]], fM(fS(f[c][P.q[k]], f[c][P.p[k]]), P.t[k]));
         for (int k = 3; k < P.nv; k++)
-            put_shade<false>(job, rowbase + (uint32_t)(k - 3), l, V3{f[0][k], f[1][k], f[2][k]},
-                             V3{f[3][k], f[4][k], f[5][k]});
+            put_shade(job, rowbase + (uint32_t)(k - 3), l, V3{f[0][k], f[1][k], f[2][k]},
+                      V3{f[3][k], f[4][k], f[5][k]});
     }
 }
 
-template <bool WIDE>
 __device__ __forceinline__ void store_edges(DgTriRec* r, const EdgeSet& e) {
     float4* d = reinterpret_cast<float4*>(r);
-    const float4 w0 = make_float4(e.A[0], e.A[1], e.A[2], e.B[0]), w1 = make_float4(e.B[1], e.B[2], e.C[0], e.C[1]);
-    const float4 w2 = make_float4(e.C[2], e.D[0], e.D[1], e.D[2]);
-    const float4 w3 = make_float4(e.den[0], e.den[1], e.den[2], __uint_as_float(e.tie));
-    if (WIDE) {
-        stg8(d, w0, w1);
-        stg8(d + 2, w2, w3);
-    } else {
-        d[0] = w0;
-        d[1] = w1;
-        d[2] = w2;
-        d[3] = w3;
-    }
+    d[0] = make_float4(e.A[0], e.A[1], e.A[2], e.B[0]);
+    d[1] = make_float4(e.B[1], e.B[2], e.C[0], e.C[1]);
+    d[2] = make_float4(e.C[2], e.D[0], e.D[1], e.D[2]);
+    d[3] = make_float4(e.den[0], e.den[1], e.den[2], __uint_as_float(e.tie));
 }
 template <bool WIDE>
 __device__ __forceinline__ void load_edges(const DgTriRec* r, EdgeSet& e) {
@@ -658,7 +635,7 @@ __device__ __forceinline__ void mat_words(const DgSegDev& sg, uint32_t mi, float
 __device__ __forceinline__ void write_record(const DgJobDev& job, DgTriRec* R, const DgSegDev& sg, uint4 tp, uint4 tuv,
                                              uint4 tnr, const EdgeSet& e, const float4 r[3], const DgFrameDev& fr,
                                              float4* Wout) {
-    store_edges<true>(R, e);
+    store_edges(R, e);
     if (Wout) {
         const float4 pa = __ldg(sg.pos + tp.x), pb = __ldg(sg.pos + tp.y), pc = __ldg(sg.pos + tp.z);
         *Wout = inv_w3(fr, V3{pa.x, pa.y, pa.z}, V3{pb.x, pb.y, pb.z}, V3{pc.x, pc.y, pc.z});
@@ -669,12 +646,15 @@ __device__ __forceinline__ void write_record(const DgJobDev& job, DgTriRec* R, c
     uint4 last;
     mat_words(sg, tp.w, mw, last, job);
     float4* d = reinterpret_cast<float4*>(R);
-    stg8(d + 4, make_float4(r[0].z, r[1].z, r[2].z, mw[0]), make_float4(u0.x, u1.x, u2.x, mw[1]));
-    stg8(d + 6, make_float4(u0.y, u1.y, u2.y, mw[2]), make_float4(n0.x, n1.x, n2.x, mw[3]));
-    stg8(d + 8, make_float4(n0.y, n1.y, n2.y, mw[4]), make_float4(n0.z, n1.z, n2.z, mw[5]));
-    const uint4 rows =
+    d[4] = make_float4(r[0].z, r[1].z, r[2].z, mw[0]);
+    d[5] = make_float4(u0.x, u1.x, u2.x, mw[1]);
+    d[6] = make_float4(u0.y, u1.y, u2.y, mw[2]);
+    d[7] = make_float4(n0.x, n1.x, n2.x, mw[3]);
+    d[8] = make_float4(n0.y, n1.y, n2.y, mw[4]);
+    d[9] = make_float4(n0.z, n1.z, n2.z, mw[5]);
+    reinterpret_cast<uint4*>(R)[10] =
         make_uint4(sg.vtx_begin + tp.x, sg.vtx_begin + tp.y, sg.vtx_begin + tp.z, __float_as_uint(mw[6]));
-    stg8(d + 10, as_float4(rows), as_float4(last));
+    reinterpret_cast<uint4*>(R)[11] = last;
 }
 
 // Triangle record of clip output o: attribute fields through the clip program;
@@ -683,7 +663,7 @@ __device__ __noinline__ void write_clip_record(const DgJobDev& job, DgTriRec* R,
                                                uint4 tuv, uint4 tnr, const EdgeSet& e, const RTri& tr,
                                                const ClipProg& P, int o, uint32_t rowbase, const DgFrameDev& fr,
                                                float4* Wout) {
-    store_edges<false>(R, e);
+    store_edges(R, e);
     if (Wout) *Wout = inv_w3(fr, P.pos[P.out[o][0]], P.pos[P.out[o][1]], P.pos[P.out[o][2]]);
     const float2 u0 = __ldg(sg.uv + tuv.x), u1 = __ldg(sg.uv + tuv.y), u2 = __ldg(sg.uv + tuv.z);
     const float4 n0 = __ldg(sg.nrm + tnr.x), n1 = __ldg(sg.nrm + tnr.y), n2 = __ldg(sg.nrm + tnr.z);
