@@ -480,7 +480,7 @@ static dg_status slot_reset(JobSlot& S) {
     return DG_OK;
 }
 
-uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L, uint64_t P) {
+uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L, bool lazy) {
     auto cap_after = [](size_t cap, const void* p, size_t need) -> size_t {
         return (cap >= need && p) ? cap : std::max(need, cap * 3 / 2);
     };
@@ -493,10 +493,11 @@ uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L
     const size_t sm = cap_after(s.small_cap, s.d_small, queue_records(T));
     const size_t qb = cap_after(s.items_cap, s.d_items, dg_items_cap(q));
     const size_t sv = cap_after(s.surv_cap, s.d_surv, std::max<uint64_t>(T, 1));
+    const size_t re = lazy ? cap_after(s.rest_cap, s.d_rest, T) : s.rest_cap;
     const size_t ro = cap_after(s.rec_of_cap, s.d_rec_of, std::max<uint64_t>(T, 1));
     const size_t tr = cap_after(s.trec_cap, s.d_trec, trec_records(T));
     return vmask * sizeof(uint16_t) + vrec * sizeof(float4) + vshade * sizeof(float4) + vmark * sizeof(uint8_t) + q * sizeof(DgQueueRec) + sm * sizeof(DgSmallRec) +
-           qb * sizeof(uint2) + (sv + ro) * sizeof(uint32_t) + tr * sizeof(DgTriRec);
+           qb * sizeof(uint2) + (sv + re + ro) * sizeof(uint32_t) + tr * sizeof(DgTriRec);
 }
 
 dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarget* targets, uint32_t n,
@@ -568,19 +569,12 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
         f.flags = s.interpolation == DG_INTERP_PERSPECTIVE ? DG_FRAME_PERSPECTIVE : 0u;
         any_persp = any_persp || f.flags != 0u;
         {
-            // At least as many opaque triangles as pixels, and a light/halfway table
-            // (32 bytes per vertex and light) beyond the L2: the small triangles get no
-            // rows and no records, and the pixels they win are shaded from the mesh.
-            // Measured without the rows alone: the 3840x2160 frame of 10M micro
-            // triangles and 4 lights gained 5% (most of its triangles win no pixel); a
-            // 256x256 frame of a 300k-triangle mesh and 1 light (a 5 MB table) lost 14%,
-            // so it keeps both. k_setup_lean has the figures without the records.
             uint64_t frame_tris = 0, frame_vtx = 0;
             for (int32_t oid : s.objects) {
                 frame_tris += c->objects[oid].ntri_opaque;
                 frame_vtx += c->objects[oid].nv;
             }
-            if (frame_tris >= tg.w * tg.h && frame_vtx * s.lights.size() * 32u >= (128ull << 20)) {
+            if (dg_frame_lazy(frame_tris, frame_vtx, s.lights.size(), tg.w * tg.h)) {
                 f.flags |= DG_FRAME_LAZY;
                 any_lazy = true;
             }

@@ -121,6 +121,18 @@ struct FrameTarget {
     uint32_t epoch;   // differs from the frame's other renders into the same cells
 };
 
+// Whether a frame of this many opaque triangles, vertices, lights and pixels gets
+// DG_FRAME_LAZY: at least as many triangles as pixels, and a light/halfway table (32
+// bytes per vertex and light) beyond the L2. The small triangles then get no rows and
+// no records, and the pixels they win are shaded from the mesh. Measured without the
+// rows alone: the 3840x2160 frame of 10M micro triangles and 4 lights gained 5% (most
+// of its triangles win no pixel); a 256x256 frame of a 300k-triangle mesh and 1 light
+// (a 5 MB table) lost 14%, so it keeps both. k_setup_lean has the figures without the
+// records.
+inline bool dg_frame_lazy(uint64_t tris, uint64_t vertices, uint64_t lights, uint64_t pixels) {
+    return tris >= pixels && vertices * lights * 32u >= (128ull << 20);
+}
+
 // Words of DgFrameDev::cells for a w x h canvas.
 inline uint64_t dg_cell_count(uint64_t w, uint64_t h) { return ((w + 31u) / 32u) * ((h + 31u) / 32u); }
 
@@ -259,8 +271,9 @@ dg_status slot_take_errors(JobSlot& s);
 // Uploads the texture table if textures were added.
 dg_status sync_tex_table(dg_ctx* c, cudaStream_t s);
 // Device bytes slot s's scratch will hold after launching a job of V vertices,
-// T triangles, L lights per vertex and P pixels (same sizing rules as launch_frames).
-uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L, uint64_t P);
+// T triangles and L lights per vertex, lazy: one of whose frames is dg_frame_lazy
+// (same sizing rules as launch_frames).
+uint64_t slot_scratch_after(const JobSlot& s, uint64_t V, uint64_t T, uint32_t L, bool lazy);
 // Builds and launches one render job over n frames on slot s (asynchronous).
 dg_status launch_frames(dg_ctx* c, JobSlot& s, Scene* const* scenes, const FrameTarget* targets, uint32_t n);
 

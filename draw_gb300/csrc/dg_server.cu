@@ -276,16 +276,19 @@ void scheduler(dg_server* s) {
             // budget covers the requests' buffers and the scratch growth of the batch
             std::vector<Request*> batch;
             uint64_t reserved = 0;  // growth of the slot's scratch this batch will cause
-            uint64_t V = 0, T = 0, P = 0;
+            uint64_t V = 0, T = 0;
             uint32_t L = 1;
+            bool lazy = false;
             const uint64_t cur = free_slot->js.scratch_bytes;
             const uint32_t cap = lane == 1 ? std::min(s->max_batch, kLargeBatch) : s->max_batch;
             while (!q.empty() && batch.size() < cap) {
                 Request* r = q.front();
                 const Object& o = s->ctx->objects[r->scene.objects[0]];
-                const uint64_t V2 = V + o.nv, T2 = T + o.ntri_opaque, P2 = P + r->scene.width * r->scene.height;
+                const uint64_t V2 = V + o.nv, T2 = T + o.ntri_opaque;
                 const uint32_t L2 = std::max<uint32_t>(L, (uint32_t)r->scene.lights.size());
-                const uint64_t after = slot_scratch_after(free_slot->js, V2, T2, L2, P2);
+                const bool lazy2 = lazy || dg_frame_lazy(o.ntri_opaque, o.nv, r->scene.lights.size(),
+                                                         r->scene.width * r->scene.height);
+                const uint64_t after = slot_scratch_after(free_slot->js, V2, T2, L2, lazy2);
                 const uint64_t grow_by = after > cur ? after - cur : 0;
                 auto pit = s->pool.find(r->size_key);
                 const bool pooled = !r->fail_alloc && pit != s->pool.end() && !pit->second.empty();
@@ -314,8 +317,8 @@ void scheduler(dg_server* s) {
                 reserved = grow_by;
                 V = V2;
                 T = T2;
-                P = P2;
                 L = L2;
+                lazy = lazy2;
                 s->peak_used = std::max(s->peak_used, s->used);
                 q.pop_front();
                 r->state = kRunning;
