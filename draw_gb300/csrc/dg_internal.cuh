@@ -432,11 +432,7 @@ struct DgLaunchCfg {
 // million 93.8 / 111; batches of 156,000 68.0 / 65.9, 169,000 67.9 / 69.1, 192,000
 // 46.7 / 44.9, 280,000 81.8 / 82.7. Blocks of 128 threads: 64 and 256 measured the
 // same or up to 2 us slower.
-#if DG_TIMELINE
-#define DG_FRONT_MAX_TRI 0u  // the timeline shows every pass as a kernel of its own
-#else
 #define DG_FRONT_MAX_TRI 131072u
-#endif
 #define DG_FRONT_THREADS 128u
 #define DG_LEAN_BLOCKS_PER_SM 6u  // one wave of k_setup_lean
 #define DG_CLIP_DEFER 512u  // k_setup_raster: clipped survivors a block sets up in its second pass

@@ -72,11 +72,24 @@ __device__ __forceinline__ void timeline_waited(int k) {
         atomicMax(&g_timeline[k][2], t);
     }
 }
+// k_front does the vertex and cull passes too: each is a point at its first block's
+// start, and the kernel itself is the setup pass.
+__device__ __forceinline__ void timeline_folded() {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const unsigned long long t = timeline_now();
+        for (int k = 0; k < 2; k++) {
+            atomicMin(&g_timeline[k][0], t);
+            atomicMax(&g_timeline[k][3], t);
+        }
+    }
+}
 #define DG_TL_BLOCK(k) TimelineBlock dg_timeline_block_(k)
 #define DG_TL_WAITED(k) timeline_waited(k)
+#define DG_TL_FOLDED() timeline_folded()
 #else
 #define DG_TL_BLOCK(k) ((void)0)
 #define DG_TL_WAITED(k) ((void)0)
+#define DG_TL_FOLDED() ((void)0)
 #endif
 
 // The plane-sign mask of a vertex: bit p: plane p has f > 0; bit 8 + p: f <= 0.
@@ -589,7 +602,9 @@ __global__ void __launch_bounds__(256) k_setup_raster(const __grid_constant__ Dg
 // entries written; without the clip program and the record it runs at three times
 // the occupancy of k_setup_raster.
 __global__ void __launch_bounds__(256, 6) k_setup_lean(const __grid_constant__ DgJobDev job) {
+    DG_TL_BLOCK(2);  // a part of the setup pass
     wait_previous_kernel();
+    DG_TL_WAITED(2);
     __shared__ uint32_t s_records;  // statistics, as in dev_setup
     if (threadIdx.x == 0) s_records = 0u;
     __syncthreads();
@@ -665,9 +680,9 @@ __global__ void __launch_bounds__(256, 6) k_setup_lean(const __grid_constant__ D
 template <class IN>
 __global__ void __launch_bounds__(DG_FRONT_THREADS) k_front(const __grid_constant__ DgJobDev job,
                                                             const __grid_constant__ IN in) {
+    DG_TL_FOLDED();
     DG_TL_BLOCK(2);
     allow_next_kernel();
-    DG_TL_WAITED(2);
     begin_job(job, in);
     auto seg = [&](uint32_t i) -> const DgSegDev& { return in.segs[i]; };
     auto frame = [&](uint32_t i) -> const DgFrameDev& { return in.frames[IN::kFrames == 1u ? 0u : i]; };

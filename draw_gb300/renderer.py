@@ -234,7 +234,7 @@ class Context:
 
     def timeline(self) -> dict:
         """dg_timeline_read (DRAW_TIMELINE builds): per kernel, microseconds after the
-        first k_vertex block's start: (first block start, first wait passed, last
+        job's first block's start: (first block start, first wait passed, last
         wait passed, last block end), None where nothing was recorded."""
         raw = (ctypes.c_uint64 * (4 * len(KERNELS)))()
         _chk(self.lib.dg_timeline_read(self.h, raw, len(raw)), "timeline")

@@ -5,8 +5,9 @@
     python -m draw_gb300.timeline torus
     python -m draw_gb300.timeline stress --tris 2000000
 
-For each kernel of the job, in microseconds after the first k_vertex block
-started: when its first block started, when its first and its last block
+For each kernel of the job, in microseconds after its first block started (a
+small frame's vertex, cull and setup passes are one kernel, shown as the setup
+pass): when its first block started, when its first and its last block
 passed the wait for the previous kernel (programmatic dependent launch), and
 when its last block finished. Each frame follows a write of 256 MiB (the L2
 flushed, as bench.py times frames); the medians over the frames are printed as

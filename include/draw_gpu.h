@@ -104,7 +104,9 @@ dg_status dg_ctx_inject_launch_failure(dg_ctx* ctx, int32_t before);
  * dg_ctx_kernel_times: the global timer (ns) when its first block started, when
  * its first and its last block passed the wait for the previous kernel, and
  * when its last block finished; 0 where nothing was recorded (a kernel that did
- * not run; a resolve pass whose tiles were all cleared before the wait).
+ * not run; a resolve pass whose tiles were all cleared before the wait). A small
+ * frame's one-kernel front is "setup_raster", and "vertex" and "cull" are points at
+ * its start; the setup of micro triangles without records counts as "setup_raster".
  * Synchronizes the context's stream and clears the record. */
 dg_status dg_timeline_read(dg_ctx* ctx, uint64_t* out, int32_t n);
 /* Launch-shape knobs of the raster passes (chosen by dg_autotune below):
