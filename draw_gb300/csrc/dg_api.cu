@@ -673,7 +673,8 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
     const unsigned traster_blocks = (unsigned)c->nsm * DG_TRASTER_BLOCKS_PER_SM;
     if (ntt) {
         const uint64_t nout = 4 * ntt;
-        if (S.tsort_cap < ntt) {
+        const bool radix = tmesh_max > DG_TSORT_MAX;  // (k_tsort needs no buffers)
+        if (radix && S.tsort_cap < ntt) {
             DG_CUDA(cudaStreamSynchronize(S.stream));
             for (int k = 0; k < 2; k++) {
                 dfree(S.d_tkey[k]);
@@ -706,7 +707,7 @@ dg_status build_job(dg_ctx* c, JobSlot& S, Scene* const* scenes, const FrameTarg
             S.dirty = false;
         }
         const uint64_t tiles = (ntt + DG_SORT_TILE - 1) / DG_SORT_TILE;
-        e = grow(S, &S.d_hist, &S.hist_cap, 256 * tiles);
+        if (radix) e = grow(S, &S.d_hist, &S.hist_cap, 256 * tiles);
         if (e) return e;
     }
     if (!B.cfg.front) e = grow(S, &S.d_surv, &S.surv_cap, std::max<uint64_t>(total_tri, 1));
