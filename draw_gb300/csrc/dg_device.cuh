@@ -255,8 +255,11 @@ __device__ __forceinline__ bool covers_nothing(float ax, float ay, float bx, flo
 // rounded operation of the edge value is monotone in x, so these pixels are one
 // side of the row; the boundary is estimated from rA (about 1/A) and then moved
 // by the exact test itself, so the result does not depend on the estimate.
-// Called for DG_EDGE_SPAN edge sets (finite values, an estimate within a few
-// pixels); [x0, x1] is the row's range, hi < lo an empty result.
+// Called for DG_EDGE_SPAN edge sets (finite values); [x0, x1] is the row's range,
+// hi < lo an empty result. The estimate is off by the rounding of the edge value over
+// |A|: a pixel or two for vertices near the canvas. With vertices millions of pixels
+// away and an edge nearly along the row it can be tens of pixels and more, which the
+// lane walks, at most through the row's range.
 __device__ __forceinline__ void row_span(const EdgeSet& e, int k, float rA, float yf, int x0, int x1, int& lo, int& hi) {
     const float by = fM(e.B[k], yf);
     const bool tie = (e.tie >> k) & 1u;

@@ -188,8 +188,8 @@ struct DgEdges {
 // normalized to a den without sign bit): coverage is then a sign test.
 #define DG_EDGE_FAST 8u
 // Set in DgEdges.tie when the barycentric divisions may use div_rcp
-// (dg_device.cuh), and when moreover the edge constants are small enough that a
-// row's covered span can be estimated to within a few pixels (row_span).
+// (dg_device.cuh), and when moreover the edge constants are small enough for
+// row_span to start from an estimate of a row's covered span.
 #define DG_EDGE_RCP 32u
 #define DG_EDGE_SPAN 64u
 // Set in rec_of for a triangle without a record whose small-list entry is the
@@ -374,9 +374,10 @@ struct DgTransparentPlan {
 // reads and writes every key six times or more in 3-kernel passes.
 #define DG_TSORT_MAX 4096u
 // k_traster: units (DG_UNIT_PX pixels) per work item, nodes a warp takes from the
-// node array at a time, resident blocks per SM (with 4, a cap of 64 registers, it
-// spills; a 1280x720 frame with 19,000 transparent triangles takes 220 us against
-// 201; with 4 or 16 units per item 201 and 217 us against 197).
+// node array at a time, resident blocks per SM (3: 80 registers and 152 bytes of
+// spill stores, 248 with the extension modes; with 4, 64 registers, a 1280x720 frame
+// with 19,000 transparent triangles took 220 us against 201, with 2 215; with 4 or 16
+// units per item 201 and 217 us against 197).
 #define DG_TITEM_UNITS 8u
 #define DG_FRAG_CHUNK 128u
 #define DG_TRASTER_BLOCKS_PER_SM 3u
@@ -387,10 +388,9 @@ constexpr uint64_t dg_frag_nodes(uint64_t n, unsigned blocks) { return n + (uint
 // The descriptors of a small job travel as a kernel parameter of its first kernel
 // instead of a host-to-device copy: that kernel reads them from its parameter and
 // writes them to job.frames and job.segs, where the later kernels of the job read
-// them. A copy before the first kernel keeps it from starting under the previous
-// job's last one: batches of 2, 10 and 28 frames, one object each, took 33.3, 73.4
-// and 92.0 us with it and take 20.7, 66.0 and 81.9 us without (the first with
-// k_front as well). A launch copies its whole parameter (at most 32,764 bytes), so
+// them. The copy is one more operation for the first kernel to follow: batches of 2,
+// 10 and 28 frames, one object each, took 33.3, 73.4 and 92.0 us with it and 20.7,
+// 66.0 and 81.9 us without (the first with k_front as well). A launch copies its whole parameter (at most 32,764 bytes), so
 // there are three sizes: a batch of 10 took 0.5 us more with twice the room.
 template <uint32_t F, uint32_t S>
 struct alignas(16) DgInlineDescT {

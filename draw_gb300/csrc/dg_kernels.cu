@@ -730,12 +730,13 @@ __device__ __forceinline__ SmallTri load_small(const DgSmallRec* s) {
 // one addition per edge and pixel); the covered pixels of all 32 are then listed together
 // and finished one per lane, so that the divisions and the keyed minimum run on
 // full warps (about a fifth of the box pixels are covered, unevenly). Measured
-// for the queue pass on 10M micro triangles and on 32 small frames: 306 and 53
-// us; with the pixels of all boxes numbered together and one per lane, 393 and
-// 57; a lane finishing its own pixels, triangles ordered by box size, 411 and 70
-// (before covers_nothing). With the edge values evaluated anew at each pixel, clip
-// outputs without area listed too (57 us of it), plain divisions (bary_fast) and a
-// load of the vertex marks per 32 (40 us), the micro frame took 264; now 170.
+// for the queue pass on 10M micro triangles and on 32 small frames, by events between
+// the kernels: 305 and 53 us; with the pixels of all boxes numbered together and one
+// per lane, 393 and 57; before these and covers_nothing, a lane finishing its own
+// pixels, triangles ordered by box size, 411 and 70. Of the micro frame's pass alone
+// (ncu), 264 us, the edge values evaluated anew at each pixel, clip outputs without
+// area listed too (57 us), plain divisions (bary_fast) and a load of the vertex marks
+// per 32 (40 us) were 94; it takes 170 now.
 __device__ __forceinline__ void raster_small_chunk(const DgJobDev& job, uint32_t first, uint32_t nsmall, float4* st,
                                                    uint16_t* list) {
     const uint32_t lane = threadIdx.x & 31u;
